@@ -99,12 +99,19 @@ __global__ void k_compress(uint32_t *parent, uint64_t n, uint64_t first, uint32_
     }
 }
 
-__global__ void k_localize(const uint32_t *parent, uint32_t *labels, uint64_t n,
-                           const uint64_t *vtx_begin, uint32_t num_graphs) {
-    for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < n;
-         v += (uint64_t)gridDim.x * blockDim.x) {
-        uint64_t g = last_le(vtx_begin, 0, num_graphs, v);
-        labels[v] = (uint32_t)(parent[v] - vtx_begin[g]);
+// Every vertex's root as an id within its graph.  The graph is searched once
+// per warp where its 32 vertices lie in one.
+__global__ void __launch_bounds__(kBlock) k_localize(const uint32_t *parent, uint64_t n, const uint64_t *vtx_begin,
+                                                     uint32_t num_graphs, uint32_t *labels) {
+    const uint64_t nwarps = (uint64_t)gridDim.x * (kBlock / 32);
+    for (uint64_t w = (blockIdx.x * (uint64_t)kBlock + threadIdx.x) >> 5; w * 32 < n; w += nwarps) {
+        const uint64_t v = w * 32 + lane_id();
+        uint64_t g = last_le(vtx_begin, 0, num_graphs, w * 32);
+        if (v >= n) continue;
+        if (w * 32 + 31 >= vtx_begin[g + 1]) g = last_le(vtx_begin, g, num_graphs, v);
+        uint32_t r = parent[v], up;
+        while ((up = parent[r]) != r) r = up;
+        labels[v] = (uint32_t)(r - vtx_begin[g]);
     }
 }
 
@@ -159,25 +166,91 @@ void cc_hook_impl(ptg_graph *g, uint32_t *d_label, RunResult &rr) {
 // RMAT and ER graphs almost every vertex is in the giant component and most
 // of the edge list is never read.
 // ---------------------------------------------------------------------------
-constexpr uint32_t kAffRounds = 2;
+constexpr uint32_t kAffFirst = 2;     // edges of every row that the first two passes link
+constexpr uint32_t kAffLong = 1024;   // edges per work item of a longer row
 
+// Every vertex hangs under its first neighbour when that one is smaller
+// (stored-order rows list hubs first, given rows their smallest id): a forest
+// without one atomic, where hooking the same edges took a root search and a
+// compare-and-swap each.
 template <class OffT>
-__global__ void k_aff_sample(const OffT *off, const uint32_t *col, uint64_t n, uint32_t r, uint32_t *parent) {
+__global__ void __launch_bounds__(kBlock) k_aff_init(const OffT *off, const uint32_t *col, uint64_t n,
+                                                     uint32_t *parent) {
     for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < n; v += (uint64_t)gridDim.x * blockDim.x) {
-        OffT b = off[v], e = off[v + 1];
-        if (e - b > (OffT)r) hook(parent, (uint32_t)v, col[b + r]);
+        const OffT b = off[v];
+        parent[v] = b < off[v + 1] ? min((uint32_t)v, col[b]) : (uint32_t)v;
     }
 }
 
-// Largest component of each graph: the majority label of 9 spread samples.
-__global__ void k_aff_giant(const uint64_t *vb, uint32_t num_graphs, const uint32_t *parent, uint32_t *giant) {
+// Roots that the first two edges of a vertex join: their parents are lowered
+// to the least of them, without a retry when several edges lower the same
+// root (k_aff_sample links what is lost).  The parents are flat before
+// (k_compress), and every value written is one that was read, so only entries
+// of roots change, by edges that are linked again later.  Without these
+// rounds the threads race in k_aff_sample to join many trees, one
+// compare-and-swap after another on the same few roots.  On a degree-grouped
+// graph nearly every vertex hangs under a hub already, whose second edge
+// leads to another hub: every 32nd warp's vertices suffice to join the hubs
+// (16 us, and k_aff_sample takes 20 instead of 47-430 us at 3 M vertices and 46 M
+// edges; all vertices would race here, 165 us, and every 256th warp's leave
+// trees, 26-47 us in k_aff_sample).  In the given order the trees are many
+// and small: two rounds over all vertices take 131 us, and k_aff_sample 41
+// instead of 733 us (512 Erdos-Renyi graphs, 4 M vertices; one round: 143 us).
+template <class OffT>
+__global__ void __launch_bounds__(kBlock) k_aff_join(const OffT *off, const uint32_t *col, uint64_t n, uint32_t every,
+                                                     uint32_t *parent) {
+    const uint64_t nwarps = (uint64_t)gridDim.x * (kBlock / 32);
+    for (uint64_t w = (blockIdx.x * (uint64_t)kBlock + threadIdx.x) >> 5; w * every * 32 < n; w += nwarps) {
+        const uint64_t v = w * every * 32 + lane_id();
+        if (v >= n) continue;
+        const OffT b = off[v], e = off[v + 1];
+        if (b == e) continue;
+        const uint32_t c0 = col[b], c1 = e - b > (OffT)1 ? col[b + 1] : c0;
+        const uint32_t r = parent[v], r0 = parent[c0], r1 = parent[c1], lo = min(r, min(r0, r1));
+        if (r != lo && lo < *(volatile const uint32_t *)&parent[r]) atomicMin(&parent[r], lo);
+        if (r0 != lo && lo < *(volatile const uint32_t *)&parent[r0]) atomicMin(&parent[r0], lo);
+        if (r1 != lo && lo < *(volatile const uint32_t *)&parent[r1]) atomicMin(&parent[r1], lo);
+    }
+}
+
+// The first two edges of every vertex linked for good.
+template <class OffT>
+__global__ void __launch_bounds__(kBlock) k_aff_sample(const OffT *off, const uint32_t *col, uint64_t n,
+                                                       uint32_t *parent) {
+    for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < n; v += (uint64_t)gridDim.x * blockDim.x) {
+        const OffT b = off[v], e = off[v + 1];
+        if (b == e) continue;
+        const uint32_t c0 = col[b], c1 = e - b > (OffT)1 ? col[b + 1] : c0;
+        if (c0 > (uint32_t)v) hook(parent, (uint32_t)v, c0);
+        if (c1 != c0) hook(parent, (uint32_t)v, c1);
+    }
+}
+
+// Largest component of each graph: the majority root of 9 spread samples,
+// marked in a bitmap.  vb == nullptr: one graph of n vertices.
+__global__ void k_aff_giant(const uint64_t *vb, uint32_t num_graphs, uint64_t n, const uint32_t *parent,
+                            uint32_t *mark) {
     for (uint32_t g = blockIdx.x * blockDim.x + threadIdx.x; g < num_graphs; g += gridDim.x * blockDim.x) {
-        uint64_t v0 = vb[g], nv = vb[g + 1] - v0;
+        uint64_t v0 = vb ? vb[g] : 0, nv = vb ? vb[g + 1] - v0 : n;
+        if (nv == 0) continue;
         uint32_t lab[9];
+#pragma unroll
         for (int i = 0; i < 9; i++) {
             uint64_t h = (uint64_t)(g + 1) * 0x9E3779B97F4A7C15ull + (uint64_t)i * 0xBF58476D1CE4E5B9ull;
             h ^= h >> 31;
-            lab[i] = nv ? parent[v0 + h % nv] : 0u;
+            lab[i] = (uint32_t)(v0 + h % nv);
+        }
+        bool moved = true;
+        while (moved) {  // the nine walks to the roots side by side
+            uint32_t up[9];
+            moved = false;
+#pragma unroll
+            for (int i = 0; i < 9; i++) up[i] = parent[lab[i]];
+#pragma unroll
+            for (int i = 0; i < 9; i++) {
+                moved |= up[i] != lab[i];
+                lab[i] = up[i];
+            }
         }
         uint32_t best = lab[0];
         int bestc = 0;
@@ -189,84 +262,125 @@ __global__ void k_aff_giant(const uint64_t *vb, uint32_t num_graphs, const uint3
                 best = lab[i];
             }
         }
-        giant[g] = best;
+        atomicOr(&mark[best >> 5], 1u << (best & 31u));
     }
 }
 
-// Link the edges from the kAffRounds-th neighbour on of every vertex outside
-// its graph's giant component.  CTAs pull 2048-edge tiles from a counter.
+// Links the edges from the kAffFirst-th on of every vertex outside its
+// graph's giant component, and points every vertex at its root (or at the
+// giant's).  Work goes by vertices: nearly all are in the giant, so a warp
+// reads 32 vertices' parents and offsets and is done, and the edge list is
+// not walked at all.  (Going by 2048-edge tiles with a row search per edge,
+// this pass read the offsets of every edge's row only to skip it: 2.13 ms of
+// a 2.8 ms RMAT-24 call, 356 us at 3 M vertices and 46 M edges.)  The edges
+// of a warp's remaining rows are dealt to its lanes evenly; rows above
+// kAffLong edges are queued in pieces for k_aff_long, so no warp walks one
+// alone.  A walk stops at the marked root even when another warp hangs that
+// root under a smaller one meanwhile: the mark decides, so two vertices that
+// skip each other's edge always share that root.
 template <class OffT>
-__global__ void __launch_bounds__(kBlock) k_aff_finish(const OffT *off, const uint32_t *col, uint64_t n, uint64_t m,
-                                                       const uint64_t *vb, uint32_t num_graphs,
-                                                       const uint32_t *giant, uint32_t *parent,
-                                                       unsigned long long *tile_counter) {
-    __shared__ OffT s_off[kTile + 2];
-    __shared__ uint8_t s_skip[kTile + 1];
-    __shared__ uint64_t s_tile;
-    uint64_t ntiles = (m + kTile - 1) / kTile;
-    while (true) {
-        if (threadIdx.x == 0) s_tile = atomicAdd(tile_counter, 1ull);
-        __syncthreads();
-        uint64_t tile = s_tile;
-        __syncthreads();
-        if (tile >= ntiles) break;
-        uint64_t t0 = tile * kTile, t1 = min(m, t0 + kTile);
-        uint64_t r0 = block_last_le(off, 0, n, t0);
-        uint64_t r1 = block_last_le(off, r0, n, t1 - 1);
-        uint64_t nrows = r1 - r0 + 1;
-        bool staged = nrows <= (uint64_t)kTile;
-        if (staged) {
-            for (uint64_t k = threadIdx.x; k <= nrows; k += kBlock) {
-                s_off[k] = off[r0 + k];
-                if (k < nrows) {
-                    uint64_t u = r0 + k;
-                    uint32_t gi = num_graphs == 1 ? 0u : (uint32_t)last_le(vb, 0, num_graphs, u);
-                    s_skip[k] = parent[u] == giant[gi];
-                }
+__global__ void __launch_bounds__(kBlock) k_aff_finish(const OffT *off, const uint32_t *col, uint64_t n,
+                                                       const uint32_t *mark, uint32_t *parent, uint2 *items,
+                                                       unsigned long long *count) {
+    const unsigned lane = lane_id();
+    const uint64_t nwarps = (uint64_t)gridDim.x * (kBlock / 32);
+    for (uint64_t w = (blockIdx.x * (uint64_t)kBlock + threadIdx.x) >> 5; w * 32 < n; w += nwarps) {
+        const uint64_t v = w * 32 + lane;
+        OffT b = 0, e = 0;
+        bool skip = true;
+        if (v < n) {
+            b = off[v];
+            e = off[v + 1];
+            const uint32_t up = parent[v];
+            uint32_t r = up;
+            skip = bit_test(mark, (uint32_t)v) || bit_test(mark, r);
+            while (!skip) {
+                const uint32_t p = parent[r];
+                if (p == r) break;
+                r = p;
+                skip = bit_test(mark, r);
             }
+            if (r != up) parent[v] = r;
         }
-        __syncthreads();
-        for (uint64_t j = t0 + threadIdx.x; j < t1; j += kBlock) {
-            uint64_t u, rs;
-            bool skip;
-            if (staged) {
-                uint64_t k = last_le(s_off, 0, nrows, j);
-                u = r0 + k;
-                rs = s_off[k];
-                skip = s_skip[k];
-            } else {
-                u = last_le(off, r0, r0 + nrows, j);
-                rs = off[u];
-                uint32_t gi = num_graphs == 1 ? 0u : (uint32_t)last_le(vb, 0, num_graphs, u);
-                skip = parent[u] == giant[gi];
-            }
-            if (skip || j - rs < kAffRounds) continue;
-            hook(parent, (uint32_t)u, __ldcs(col + j));
+        const uint64_t rem = !skip && e - b > (OffT)kAffFirst ? (uint64_t)(e - b) - kAffFirst : 0;
+        unsigned longs = __ballot_sync(0xffffffffu, rem > kAffLong);
+        while (longs) {
+            const int src = __ffs(longs) - 1;
+            longs &= longs - 1;
+            const uint64_t pieces = (__shfl_sync(0xffffffffu, rem, src) + kAffLong - 1) / kAffLong;
+            unsigned long long at = 0;
+            if (lane == 0) at = atomicAdd(count, (unsigned long long)pieces);
+            at = __shfl_sync(0xffffffffu, at, 0);
+            for (uint64_t i = lane; i < pieces; i += 32) items[at + i] = make_uint2((uint32_t)(w * 32) + src, (uint32_t)i);
         }
-        __syncthreads();
+        const uint32_t cnt = rem > kAffLong ? 0u : (uint32_t)rem;
+        uint32_t incl = cnt;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= (unsigned)o) incl += y;
+        }
+        const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
+        for (uint32_t t0 = 0; t0 < total; t0 += 32) {  // warp-uniform bound
+            const uint32_t t = min(t0 + lane, total - 1);
+            uint32_t src = 0;  // first lane whose inclusive sum exceeds t
+#pragma unroll
+            for (uint32_t step = 16; step > 0; step >>= 1)
+                if (__shfl_sync(0xffffffffu, incl, src + step - 1) <= t) src += step;
+            const uint32_t at = t - (__shfl_sync(0xffffffffu, incl, src) - __shfl_sync(0xffffffffu, cnt, src));
+            const OffT base = __shfl_sync(0xffffffffu, b, src);
+            if (t0 + lane < total) hook(parent, (uint32_t)(w * 32) + src, __ldcs(col + base + kAffFirst + at));
+        }
     }
 }
 
-// The whole Afforest sequence on a resident CSR of one or more graphs.
+// The pieces that k_aff_finish queued, a warp each.
+template <class OffT>
+__global__ void __launch_bounds__(kBlock) k_aff_long(const OffT *off, const uint32_t *col, const uint2 *items,
+                                                     const unsigned long long *count, uint32_t *parent) {
+    const uint64_t total = *count, nwarps = (uint64_t)gridDim.x * (kBlock / 32);
+    for (uint64_t i = (blockIdx.x * (uint64_t)kBlock + threadIdx.x) >> 5; i < total; i += nwarps) {
+        const uint2 it = items[i];
+        const OffT b = off[it.x] + (OffT)kAffFirst + (OffT)it.y * (OffT)kAffLong, e = off[(uint64_t)it.x + 1];
+        const OffT end = e - b > (OffT)kAffLong ? b + (OffT)kAffLong : e;
+        for (OffT k = b + lane_id(); k < end; k += 32) hook(parent, it.x, __ldcs(col + k));
+    }
+}
+
+// The Afforest sequence up to the last link, on a resident CSR of one or
+// more graphs; the caller's last pass walks the remaining parents.  `grouped`:
+// vertices in degree order, rows listing hubs first (relabel.cu).
 template <class OffT>
 void afforest(ptg_ctx *ctx, const OffT *off, const uint32_t *col, uint64_t n, uint64_t m, const uint64_t *d_vb,
-              uint32_t num_graphs, uint32_t *parent, uint32_t *d_giant, unsigned long long *d_counter) {
+              uint32_t num_graphs, bool grouped, uint32_t *parent) {
     cudaStream_t st = ctx->stream;
+    Workspace &ws = ctx->ws;
     const int sms = ctx->sm_count;
-    int vgrid = grid_for(n, kBlock, sms * 8);
-    launch(ctx, "k_iota", k_iota, vgrid, kBlock, 0, st, parent, n, (uint64_t)0);
-    for (uint32_t r = 0; r < kAffRounds; r++) {
-        launch(ctx, "k_aff_sample", k_aff_sample<OffT>, vgrid, kBlock, 0, st, off, col, n, r, parent);
+    const uint64_t words = (n + 31) / 32;
+    ws.bm[0].ensure(words * 4);              // the marked roots
+    ws.scan.ensure((m / (kAffLong / 2) + 1) * sizeof(uint2));  // a row has at most 2 pieces per kAffLong edges
+    ws.bsum.ensure(1024 * 8);
+    uint32_t *mark = ws.bm[0].as<uint32_t>();
+    uint2 *items = ws.scan.as<uint2>();
+    unsigned long long *count = ws.bsum.as<unsigned long long>();
+    const int vgrid = grid_for(n, kBlock, sms * 8);
+    PTG_CUDA_TRY(cudaMemsetAsync(mark, 0, words * 4, st));
+    PTG_CUDA_TRY(cudaMemsetAsync(count, 0, 8, st));
+    launch(ctx, "k_aff_init", k_aff_init<OffT>, vgrid, kBlock, 0, st, off, col, n, parent);
+    launch(ctx, "k_compress", k_compress, vgrid, kBlock, 0, st, parent, n, (uint64_t)0, 0u);
+    const uint32_t every = grouped ? 32u : 1u;
+    for (int r = 0; r < (grouped ? 1 : 2); r++) {
+        launch(ctx, "k_aff_join", k_aff_join<OffT>, grid_for(n / every + 1, kBlock, sms * 8), kBlock, 0, st, off, col,
+               n, every, parent);
         launch(ctx, "k_compress", k_compress, vgrid, kBlock, 0, st, parent, n, (uint64_t)0, 0u);
     }
-    launch(ctx, "k_aff_giant", k_aff_giant, grid_for(num_graphs, kBlock, sms * 4), kBlock, 0, st, d_vb, num_graphs,
-           (const uint32_t *)parent, d_giant);
-    PTG_CUDA_TRY(cudaMemsetAsync(d_counter, 0, 8, st));
-    int occ = 0;
-    PTG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_aff_finish<OffT>, kBlock, 0));
-    launch(ctx, "k_aff_finish", k_aff_finish<OffT>, std::max(1, occ) * sms, kBlock, 0, st, off, col, n, m, d_vb,
-           num_graphs, (const uint32_t *)d_giant, parent, d_counter);
-    launch(ctx, "k_compress", k_compress, vgrid, kBlock, 0, st, parent, n, (uint64_t)0, 0u);
+    launch(ctx, "k_aff_sample", k_aff_sample<OffT>, vgrid, kBlock, 0, st, off, col, n, parent);
+    launch(ctx, "k_aff_giant", k_aff_giant, grid_for(num_graphs, 64, sms * 4), 64, 0, st, d_vb, num_graphs, n,
+           (const uint32_t *)parent, mark);
+    launch(ctx, "k_aff_finish", k_aff_finish<OffT>, vgrid, kBlock, 0, st, off, col, n, (const uint32_t *)mark, parent,
+           items, count);
+    launch(ctx, "k_aff_long", k_aff_long<OffT>, grid_for(m / kAffLong + 1, kBlock / 32, sms * 8), kBlock, 0, st, off,
+           col, (const uint2 *)items, (const unsigned long long *)count, parent);
     PTG_CUDA_TRY(cudaGetLastError());
 }
 
@@ -283,18 +397,15 @@ void run_cc_hook(ptg_graph *g, uint32_t *d_label, RunResult &rr) {
             ws.relab[1].ensure(g->n * 4);
             d_label = ws.relab[0].as<uint32_t>();
         }
-        ws.bsum.ensure(1024 * 8);
-        uint64_t *d_vb = ws.bsum.as<uint64_t>();
-        uint32_t *d_giant = reinterpret_cast<uint32_t *>(d_vb + 2);
-        unsigned long long *d_counter = reinterpret_cast<unsigned long long *>(d_vb + 4);
-        uint64_t vb[2] = {0, g->n};
-        PTG_CUDA_TRY(cudaMemcpyAsync(d_vb, vb, 16, cudaMemcpyHostToDevice, g->ctx->stream));
         if (g->off64)
             afforest<unsigned long long>(g->ctx, g->d_off.as<unsigned long long>(), g->d_col.as<uint32_t>(), g->n,
-                                         g->m, d_vb, 1, d_label, d_giant, d_counter);
+                                         g->m, nullptr, 1, g->relabeled, d_label);
         else
-            afforest<uint32_t>(g->ctx, g->d_off.as<uint32_t>(), g->d_col.as<uint32_t>(), g->n, g->m, d_vb, 1,
-                               d_label, d_giant, d_counter);
+            afforest<uint32_t>(g->ctx, g->d_off.as<uint32_t>(), g->d_col.as<uint32_t>(), g->n, g->m, nullptr, 1,
+                               g->relabeled, d_label);
+        if (!g->relabeled)
+            launch(g->ctx, "k_compress", k_compress, grid_for(g->n, kBlock, g->ctx->sm_count * 8), kBlock, 0,
+                   g->ctx->stream, d_label, g->n, (uint64_t)0, 0u);
         if (g->relabeled) cc_labels_out(g, d_label, ws.relab[1].as<uint32_t>(), out);
         rr.edges_relaxed = g->m;
         rr.iterations = 1;
@@ -311,27 +422,31 @@ void run_cc_batch(ptg_ctx *ctx, uint32_t num_graphs, const uint64_t *vtx_begin,
     uint64_t n = vtx_begin[num_graphs];
     uint64_t m = offsets[n];
     PTG_REQUIRE(n < 0xFFFFFFFFull, PTG_ERR_INVALID, "batched CC needs fewer than 2^32 vertices in total");
-    DevBuf d_off, d_col, d_parent, d_vb, d_counter, d_giant;
-    d_off.ensure((n + 1) * 8);
-    d_col.ensure(std::max<uint64_t>(m, 1) * 4);
-    d_parent.ensure(n * 4);
-    d_vb.ensure((num_graphs + 1) * 8);
-    d_counter.ensure(8);
-    d_giant.ensure((uint64_t)num_graphs * 4);
-    PTG_CUDA_TRY(cudaMemcpyAsync(d_off.p, offsets, (n + 1) * 8, cudaMemcpyHostToDevice, st));
-    if (m) PTG_CUDA_TRY(cudaMemcpyAsync(d_col.p, col, m * 4, cudaMemcpyHostToDevice, st));
-    PTG_CUDA_TRY(cudaMemcpyAsync(d_vb.p, vtx_begin, (num_graphs + 1) * 8, cudaMemcpyHostToDevice, st));
+    // one block for the uploaded CSR and the labels (of at least the size
+    // that the block cache keeps: small batches don't pay for a cudaMalloc
+    // and a cudaFree per array and call)
+    auto up = [](uint64_t x) { return (x + 255) & ~(uint64_t)255; };
+    const uint64_t o_col = up((n + 1) * 8), o_parent = o_col + up(m * 4), o_vb = o_parent + up(n * 4);
+    DevBuf block;
+    block.ensure(std::max<uint64_t>(1ull << 20, o_vb + (num_graphs + 1) * 8ull));
+    char *base = block.as<char>();
+    auto *d_off = reinterpret_cast<unsigned long long *>(base);
+    auto *d_col = reinterpret_cast<uint32_t *>(base + o_col);
+    auto *d_parent = reinterpret_cast<uint32_t *>(base + o_parent);
+    auto *d_vb = reinterpret_cast<uint64_t *>(base + o_vb);
+    auto *d_labels = reinterpret_cast<uint32_t *>(base);  // over the offsets, read by then
+    PTG_CUDA_TRY(cudaMemcpyAsync(d_off, offsets, (n + 1) * 8, cudaMemcpyHostToDevice, st));
+    if (m) PTG_CUDA_TRY(cudaMemcpyAsync(d_col, col, m * 4, cudaMemcpyHostToDevice, st));
+    PTG_CUDA_TRY(cudaMemcpyAsync(d_vb, vtx_begin, (num_graphs + 1) * 8, cudaMemcpyHostToDevice, st));
     PTG_CUDA_TRY(cudaEventRecord(ctx->ev0, st));
-    // one Afforest pass over the concatenated CSR: a single persistent launch
-    // links the remaining edges of every graph, however uneven the graphs are
-    afforest<unsigned long long>(ctx, d_off.as<unsigned long long>(), d_col.as<uint32_t>(), n, m,
-                                 d_vb.as<uint64_t>(), num_graphs, d_parent.as<uint32_t>(), d_giant.as<uint32_t>(),
-                                 d_counter.as<unsigned long long>());
+    // one Afforest pass over the concatenated CSR links the edges of every
+    // graph, however uneven the graphs are
+    afforest<unsigned long long>(ctx, d_off, d_col, n, m, d_vb, num_graphs, false, d_parent);
     launch(ctx, "k_localize", k_localize, grid_for(n, kBlock, sms * 8), kBlock, 0, st,
-           d_parent.as<uint32_t>(), d_parent.as<uint32_t>(), n, d_vb.as<uint64_t>(), num_graphs);
+           (const uint32_t *)d_parent, n, (const uint64_t *)d_vb, num_graphs, d_labels);
     PTG_CUDA_TRY(cudaGetLastError());
     PTG_CUDA_TRY(cudaEventRecord(ctx->ev1, st));
-    PTG_CUDA_TRY(cudaMemcpyAsync(labels, d_parent.p, n * 4, cudaMemcpyDeviceToHost, st));
+    PTG_CUDA_TRY(cudaMemcpyAsync(labels, d_labels, n * 4, cudaMemcpyDeviceToHost, st));
     PTG_CUDA_TRY(cudaStreamSynchronize(st));
     float ms = 0;
     cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);

@@ -411,6 +411,6 @@ void map_sources_dev(ptg_graph *g, uint32_t *d_ids, uint32_t k);
 uint32_t map_source_host(ptg_graph *g, uint32_t src);
 void unpermute_u32(ptg_graph *g, const uint32_t *tmp, uint32_t *out, uint32_t rows);
 void unpermute_f32(ptg_graph *g, const float *tmp, float *out);
-void cc_labels_out(ptg_graph *g, const uint32_t *lab, uint32_t *scratch, uint32_t *out);
+void cc_labels_out(ptg_graph *g, uint32_t *lab, uint32_t *scratch, uint32_t *out);
 
 }  // namespace ptg

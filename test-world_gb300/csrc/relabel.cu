@@ -361,14 +361,32 @@ __global__ void __launch_bounds__(kBlock) k_unpermute(const T *tmp, const uint32
     }
 }
 
-// component label (a new id shared by the component) -> minimum caller id.
-// The read before the atomic keeps the giant component's vertices from all
-// hitting one address: once its minimum is in, they see it and skip.
-__global__ void __launch_bounds__(kBlock) k_cc_minold(const uint32_t *lab, const uint32_t *perm, uint64_t n,
+// Component (the root that a vertex's parents lead to, a new id) -> minimum
+// caller id, with every vertex pointed at its root on the way.  Vertices of
+// the component of vertex 0 (the highest degree: nearly always the giant)
+// meet in registers and then once per CTA: hundreds of thousands of threads
+// reading the not yet lowered minimum and then all sending an atomic to that
+// one address took 164 us, whatever the graph's size.
+__global__ void __launch_bounds__(kBlock) k_cc_minold(uint32_t *lab, const uint32_t *perm, uint64_t n,
                                                       uint32_t *minold) {
+    __shared__ uint32_t s_min[kBlock / 32];
+    uint32_t giant = lab[0], up;
+    while ((up = lab[giant]) != giant) giant = up;
+    uint32_t least = 0xFFFFFFFFu;
     for (uint64_t x = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; x < n; x += (uint64_t)gridDim.x * blockDim.x) {
-        uint32_t l = lab[x], o = perm[x];
-        if (o < *(volatile const uint32_t *)&minold[l]) atomicMin(&minold[l], o);
+        const uint32_t first = lab[x], o = perm[x];
+        uint32_t l = first;
+        while ((up = lab[l]) != l) l = up;
+        if (l != first) lab[x] = l;
+        if (l == giant) least = min(least, o);
+        else if (o < *(volatile const uint32_t *)&minold[l]) atomicMin(&minold[l], o);
+    }
+    least = __reduce_min_sync(0xffffffffu, least);
+    if (lane_id() == 0) s_min[threadIdx.x >> 5] = least;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int i = 1; i < kBlock / 32; i++) least = min(least, s_min[i]);
+        if (least != 0xFFFFFFFFu) atomicMin(&minold[giant], least);
     }
 }
 
@@ -669,13 +687,14 @@ void unpermute_f32(ptg_graph *g, const float *tmp, float *out) {
            g->ctx->stream, tmp, (const uint32_t *)g->d_newid.p, g->n, 1u, out);
 }
 
-void cc_labels_out(ptg_graph *g, const uint32_t *lab, uint32_t *scratch, uint32_t *out) {
+// `lab`: parents that lead to each component's root (flattened here).
+void cc_labels_out(ptg_graph *g, uint32_t *lab, uint32_t *scratch, uint32_t *out) {
     ptg_ctx *ctx = g->ctx;
     cudaStream_t st = ctx->stream;
     int grid = grid_for(g->n, kBlock, ctx->sm_count * 8);
     PTG_CUDA_TRY(cudaMemsetAsync(scratch, 0xFF, g->n * 4, st));
     launch(ctx, "k_cc_minold", k_cc_minold, grid, kBlock, 0, st, lab, (const uint32_t *)g->d_perm.p, g->n, scratch);
-    launch(ctx, "k_cc_out", k_cc_out, grid, kBlock, 0, st, lab, (const uint32_t *)g->d_perm.p,
+    launch(ctx, "k_cc_out", k_cc_out, grid, kBlock, 0, st, (const uint32_t *)lab, (const uint32_t *)g->d_perm.p,
            (const uint32_t *)scratch, g->n, out);
 }
 
