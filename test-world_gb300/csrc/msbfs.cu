@@ -33,13 +33,11 @@ typedef unsigned long long u64;
 // MS-BFS, W mask words per vertex (layout M[v*W + w])
 // ---------------------------------------------------------------------------
 template <int W>
-__global__ void k_msb_seed(const uint32_t *srcs, uint32_t k, u64 *F, u64 *S, uint32_t *out, uint64_t n,
-                           uint32_t base) {
+__global__ void k_msb_seed(const uint32_t *srcs, uint32_t k, u64 *F, u64 *S) {
     for (uint32_t i = threadIdx.x; i < k; i += blockDim.x) {
         uint32_t s = srcs[i];
         atomicOr(&F[(uint64_t)s * W + i / 64], 1ull << (i % 64));
         atomicOr(&S[(uint64_t)s * W + i / 64], 1ull << (i % 64));
-        out[(uint64_t)i * n + s] = base;
     }
 }
 
@@ -60,24 +58,6 @@ __global__ void __launch_bounds__(kBlock) k_msb_queue(const u64 *M, uint64_t n, 
     }
     degsum = block_reduce_sum(degsum);
     if (threadIdx.x == 0 && degsum) atomicAdd(&ctl->m_unvisited, degsum);
-}
-
-// Write level `val` into out[s*n + v] for every source bit s in nb; the warp
-// loops over the union of its lanes' bits so each store is coalesced.
-template <int W>
-__device__ __forceinline__ void msb_write_levels(uint32_t *out, uint64_t n, uint64_t v, bool valid,
-                                                 const u64 (&nb)[W], uint32_t val) {
-#pragma unroll
-    for (int w = 0; w < W; w++) {
-        u64 any = nb[w];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) any |= __shfl_xor_sync(0xffffffffu, any, o);
-        while (any) {
-            int i = __ffsll((long long)any) - 1;
-            any &= any - 1;
-            if (valid && ((nb[w] >> i) & 1ull)) out[(uint64_t)(w * 64 + i) * n + v] = val;
-        }
-    }
 }
 
 // Push level: every edge (u -> v) of the frontier ORs F[u] into N[v].
@@ -148,41 +128,105 @@ __device__ __forceinline__ void live_or(u64 *live_next, const u64 (&nb)[W]) {
     }
 }
 
-// After a push: N[v] &= ~S[v], S |= N, levels written, next queue built.
+// After a level: N[v] &= ~S[v], S |= N, next queue built.
 template <class OffT, int W>
-__global__ void __launch_bounds__(kBlock) k_msb_update(uint64_t n, const OffT *off, u64 *N, u64 *S,
-                                                       uint32_t *out, uint32_t val, uint32_t *q, TravCtl *ctl,
-                                                       u64 *live_next) {
+__global__ void __launch_bounds__(kBlock) k_msb_update(uint64_t n, const OffT *off, u64 *N, u64 *S, uint32_t *q,
+                                                       TravCtl *ctl, u64 *live_next) {
     unsigned long long degsum = 0;
-    uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    uint64_t span = (n + 31) / 32 * 32;
-    for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < span; v += stride) {
-        bool valid = v < n;
-        u64 nb[W];
+    u64 live[W];
+#pragma unroll
+    for (int w = 0; w < W; w++) live[w] = 0;
+    for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < n; v += (uint64_t)gridDim.x * blockDim.x) {
+        u64 x[W];
+        load_mask<W>(N + v * W, x);
         bool any = false;
 #pragma unroll
+        for (int w = 0; w < W; w++) any |= x[w] != 0ull;
+        if (!any) continue;
+        u64 s[W];
+        load_mask<W>(S + v * W, s);
+        any = false;
+#pragma unroll
         for (int w = 0; w < W; w++) {
-            nb[w] = 0;
-            if (valid) {
-                u64 x = N[v * W + w];
-                if (x) {
-                    u64 s = S[v * W + w];
-                    nb[w] = x & ~s;
-                    N[v * W + w] = nb[w];
-                    if (nb[w]) S[v * W + w] = s | nb[w];
-                }
-            }
-            any |= nb[w] != 0ull;
+            const u64 nb = x[w] & ~s[w];
+            if (nb != x[w]) N[v * W + w] = nb;
+            if (nb) S[v * W + w] = s[w] | nb;
+            live[w] |= nb;
+            any |= nb != 0ull;
         }
-        msb_write_levels<W>(out, n, v, valid, nb, val);
-        live_or<W>(live_next, nb);
         if (any) {
             degsum += (unsigned long long)(off[v + 1] - off[v]);
             warp_append(q, &ctl->next_tail, (unsigned)n, &ctl->error, (uint32_t)v);
         }
     }
+    __syncwarp();
+    live_or<W>(live_next, live);
     degsum = block_reduce_sum(degsum);
     if (threadIdx.x == 0 && degsum) atomicAdd(&ctl->m_unvisited, degsum);
+}
+
+// The frontier masks of up to kMsHist consecutive levels.
+constexpr int kMsHist = 12;
+static_assert(kMsHist <= 16, "a level's position has four bits");
+struct MsHist {
+    const u64 *m[kMsHist];
+};
+
+// Rows out of the kept levels: out[s*n + v] = level0 + l for the level l whose
+// mask holds source s at v (at newid[v] on a regrouped graph).  FIRST: every
+// word is written, unreached where no level has it; else only the found ones.
+// The position of a source's level is put together from four words of bits
+// (levels with bit 0..3 of their position set), so a source takes a few
+// instructions a vertex however many levels there are.  Bound by the rows'
+// stores: 4.3 GB in 1.0 ms for 256 sources on 4.2 M vertices.  The rows are
+// written once: writing them level by level (a fill, scattered words per
+// level, then a gather to the caller's ids) moved them five times and took
+// 5.7 of that call's 8.8 ms (now 4.7).  Twelve levels are what an RMAT search
+// needs (9-10); with eight the second pass over the rows cost another 0.1 ms.
+template <int W, bool FIRST>
+__global__ void __launch_bounds__(kBlock) k_msb_levels(MsHist h, int cnt, uint64_t n, uint32_t k,
+                                                       const uint32_t *newid, uint32_t level0, uint32_t *out) {
+    for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < n; v += (uint64_t)gridDim.x * blockDim.x) {
+        const uint64_t x = newid ? newid[v] : v;
+        u64 any[W], p0[W], p1[W], p2[W], p3[W];
+#pragma unroll
+        for (int w = 0; w < W; w++) any[w] = p0[w] = p1[w] = p2[w] = p3[w] = 0ull;
+#pragma unroll
+        for (int l = 0; l < kMsHist; l++) {
+            if (l >= cnt) break;
+            u64 m[W];
+            load_mask<W>(h.m[l] + x * W, m);
+#pragma unroll
+            for (int w = 0; w < W; w++) {
+                any[w] |= m[w];
+                if (l & 1) p0[w] |= m[w];
+                if (l & 2) p1[w] |= m[w];
+                if (l & 4) p2[w] |= m[w];
+                if (l & 8) p3[w] |= m[w];
+            }
+        }
+        uint32_t *o = out + v;
+#pragma unroll
+        for (int hw = 0; hw < 2 * W; hw++) {
+            const int sh = (hw & 1) * 32;
+            const uint32_t a = (uint32_t)(any[hw / 2] >> sh), b0 = (uint32_t)(p0[hw / 2] >> sh);
+            const uint32_t b1 = (uint32_t)(p1[hw / 2] >> sh), b2 = (uint32_t)(p2[hw / 2] >> sh);
+            const uint32_t b3 = (uint32_t)(p3[hw / 2] >> sh);
+            const uint32_t left = k > (uint32_t)hw * 32 ? min(32u, k - (uint32_t)hw * 32) : 0u;
+            if (!FIRST && !a) {
+                o += (uint64_t)left * n;
+                continue;
+            }
+#pragma unroll 8
+            for (uint32_t s = 0; s < left; s++) {
+                const uint32_t at = ((b0 >> s) & 1u) | (((b1 >> s) & 1u) << 1) | (((b2 >> s) & 1u) << 2) |
+                                    (((b3 >> s) & 1u) << 3);
+                const bool found = (a >> s) & 1u;
+                if (FIRST || found) __stcs(o, found ? level0 + at : PTG_UNREACHED);
+                o += n;
+            }
+        }
+    }
 }
 
 // Pull level (symmetric graphs): N[v] = (OR of F over v's neighbours) & ~S[v],
@@ -499,12 +543,9 @@ void ms_scan(ptg_ctx *ctx, Workspace &ws, const OffT *off, uint64_t m, uint64_t 
 }
 
 template <class OffT>
-void ms_prepare(ptg_graph *g, uint64_t mask_bytes) {
+void ms_prepare(ptg_graph *g) {
     Workspace &ws = g->ctx->ws;
     uint64_t n = g->n, m = g->m;
-    ws.ms[0].ensure(mask_bytes);
-    ws.ms[1].ensure(mask_bytes);
-    ws.ms[2].ensure(mask_bytes);
     ws.q[0].ensure(n * 4);
     ws.q[1].ensure(n * 4);
     ws.scan.ensure((n + 1) * sizeof(OffT));
@@ -601,17 +642,30 @@ void msbfs_impl(ptg_graph *g, const uint32_t *h_srcs, uint32_t k, uint32_t *d_ro
     const OffT *off = g->d_off.as<OffT>();
     const uint32_t *col = g->d_col.as<uint32_t>();
     uint32_t base = (flags & PTG_LEVEL_ZERO_BASED) ? 0u : 1u;
-    ms_prepare<OffT>(g, n * 8 * W);
+    ms_prepare<OffT>(g);
+    // ms[0]: the levels' frontier masks, as many as there is memory for (two
+    // at least: a level and the next); ms[1]: sources seen per vertex
+    const uint64_t mask_words = (n * W + 31) / 32 * 32, mask_bytes = mask_words * 8;
+    ws.ms[1].ensure(mask_bytes);
+    int hist = kMsHist;
+    try {
+        ws.ms[0].ensure(hist * mask_bytes);
+    } catch (const Error &e) {
+        if (e.status != PTG_ERR_OOM) throw;
+        cudaGetLastError();
+        hist = 2;
+        ws.ms[0].ensure(hist * mask_bytes);
+    }
     if (g->symmetric && !g->pull_items_built) build_pull_items<OffT>(g);
-    u64 *M0 = ws.ms[0].as<u64>(), *M1 = ws.ms[1].as<u64>(), *S = ws.ms[2].as<u64>();
+    u64 *S = ws.ms[1].as<u64>();
+    MsHist h{};
+    for (int i = 0; i < hist; i++) h.m[i] = ws.ms[0].as<u64>() + i * mask_words;
     unsigned long long *bsum = ws.bsum.as<unsigned long long>();
     uint32_t *d_srcs = reinterpret_cast<uint32_t *>(bsum + 1024);
     u64 *d_all = reinterpret_cast<u64 *>(d_srcs + 256);
     TravCtl *d_ctl = ws.ctl.as<TravCtl>();
-    PTG_CUDA_TRY(cudaMemsetAsync(d_rows, 0xFF, (uint64_t)k * n * 4, st));
     PTG_CUDA_TRY(cudaMemsetAsync(S, 0, n * 8 * W, st));
-    PTG_CUDA_TRY(cudaMemsetAsync(M0, 0, n * 8 * W, st));
-    PTG_CUDA_TRY(cudaMemsetAsync(M1, 0, n * 8 * W, st));
+    PTG_CUDA_TRY(cudaMemsetAsync((void *)h.m[0], 0, n * 8 * W, st));
     u64 all[W];
     for (int w = 0; w < W; w++) {
         int bits = std::max(0, std::min(64, (int)k - 64 * w));
@@ -619,17 +673,32 @@ void msbfs_impl(ptg_graph *g, const uint32_t *h_srcs, uint32_t k, uint32_t *d_ro
     }
     PTG_CUDA_TRY(cudaMemcpyAsync(d_srcs, h_srcs, k * 4, cudaMemcpyHostToDevice, st));
     map_sources_dev(g, d_srcs, k);
-    PTG_CUDA_TRY(cudaMemcpyAsync(d_all, all, sizeof(all), cudaMemcpyHostToDevice, st));
-    launch(ctx, "k_msb_seed", k_msb_seed<W>, 1, 256, 0, st, (const uint32_t *)d_srcs, k, M0, S, d_rows, n, base);
+    launch(ctx, "k_msb_seed", k_msb_seed<W>, 1, 256, 0, st, (const uint32_t *)d_srcs, k, (u64 *)h.m[0], S);
     TravCtl init{};
     PTG_CUDA_TRY(cudaMemcpyAsync(d_ctl, &init, sizeof(TravCtl), cudaMemcpyHostToDevice, st));
     int vgrid = grid_for(n, kBlock, sms * 8);
-    launch(ctx, "k_msb_queue", k_msb_queue<OffT, W>, vgrid, kBlock, 0, st, (const u64 *)M0, n, off,
+    launch(ctx, "k_msb_queue", k_msb_queue<OffT, W>, vgrid, kBlock, 0, st, h.m[0], n, off,
            ws.q[1].as<uint32_t>(), d_ctl);
     uint64_t F, Eact, E;
     ms_next(ctx, ws, F, Eact, E);
-    uint32_t level = base;
-    int cur = 0;
+    // the kept levels: h.m[0] is level `level0`, h.m[cnt - 1] the current
+    // frontier, and the first `written` of them are in the rows already
+    uint32_t level0 = base;
+    int cnt = 1, written = 0, round = 0;
+    bool first = true;
+    auto write_levels = [&] {
+        MsHist part{};
+        for (int i = written; i < cnt; i++) part.m[i - written] = h.m[i];
+        const uint32_t *newid = g->relabeled ? g->d_newid.as<uint32_t>() : nullptr;
+        const int grid = grid_for(n, kBlock, sms * 8);
+        if (first)
+            launch(ctx, "k_msb_levels", k_msb_levels<W, true>, grid, kBlock, 0, st, part, cnt - written, n, k, newid,
+                   level0 + (uint32_t)written, d_rows);
+        else
+            launch(ctx, "k_msb_levels", k_msb_levels<W, false>, grid, kBlock, 0, st, part, cnt - written, n, k, newid,
+                   level0 + (uint32_t)written, d_rows);
+        first = false;
+    };
     // live[c]: OR of every frontier mask of the current level (the sources
     // still expanding); the seed frontier holds all of them.
     u64 *d_live[2] = {d_all + 4, d_all + 8};
@@ -638,31 +707,40 @@ void msbfs_impl(ptg_graph *g, const uint32_t *h_srcs, uint32_t k, uint32_t *d_ro
     while (F > 0) {
         if (rr.iterations >= max_rounds) throw Error{PTG_ERR_TIMEOUT, "iteration limit reached"};
         rr.iterations++;
-        u64 *Mc = cur ? M1 : M0, *Mn = cur ? M0 : M1;
-        PTG_CUDA_TRY(cudaMemsetAsync(d_live[cur ^ 1], 0, 8 * W, st));
+        if (cnt == hist) {  // full: the rows take the kept levels, the frontier stays
+            write_levels();
+            std::swap(h.m[0], h.m[cnt - 1]);
+            level0 += (uint32_t)cnt - 1;
+            cnt = written = 1;
+        }
+        const u64 *Mc = h.m[cnt - 1];
+        u64 *Mn = (u64 *)h.m[cnt];
+        PTG_CUDA_TRY(cudaMemsetAsync(d_live[round ^ 1], 0, 8 * W, st));
         bool pull = g->symmetric && Eact * 10 > m;
         PTG_CUDA_TRY(cudaMemsetAsync(Mn, 0, n * 8 * W, st));
         if (pull) {
             launch(ctx, "k_msb_pull_small", k_msb_pull_small<OffT, W>, vgrid, kBlock, 0, st, n, off, col,
-                   (const u64 *)Mc, (const u64 *)S, Mn, (const u64 *)d_live[cur], g->pull_small);
+                   Mc, (const u64 *)S, Mn, (const u64 *)d_live[round], g->pull_small);
             if (g->n_pull_items)
                 launch(ctx, "k_msb_pull_big", k_msb_pull_big<OffT, W>, sms * 8, kBlock, 0, st,
-                       (const uint2 *)g->d_pull_items.p, g->n_pull_items, off, col, (const u64 *)Mc,
-                       (const u64 *)S, Mn, (const u64 *)d_live[cur], g->pull_chunk);
+                       (const uint2 *)g->d_pull_items.p, g->n_pull_items, off, col, Mc,
+                       (const u64 *)S, Mn, (const u64 *)d_live[round], g->pull_chunk);
         } else {
             ms_scan<OffT>(ctx, ws, off, m, F, d_ctl);
             launch(ctx, "k_msb_push", k_msb_push<OffT, W>, sms * 8, kBlock, 0, st, (const uint32_t *)ws.q[0].p,
                    (const OffT *)ws.scan.p, (const OffT *)ws.rowstart.p, (const uint32_t *)ws.tiles.p, col,
-                   (const u64 *)Mc, (const u64 *)S, Mn, (const TravCtl *)d_ctl);
+                   Mc, (const u64 *)S, Mn, (const TravCtl *)d_ctl);
         }
-        launch(ctx, "k_msb_update", k_msb_update<OffT, W>, vgrid, kBlock, 0, st, n, off, Mn, S, d_rows,
-               level + 1, ws.q[1].as<uint32_t>(), d_ctl, d_live[cur ^ 1]);
+        launch(ctx, "k_msb_update", k_msb_update<OffT, W>, vgrid, kBlock, 0, st, n, off, Mn, S,
+               ws.q[1].as<uint32_t>(), d_ctl, d_live[round ^ 1]);
         PTG_CUDA_TRY(cudaGetLastError());
         ms_next(ctx, ws, F, Eact, E);
         rr.edges_relaxed += pull ? 0 : E;
-        cur ^= 1;
-        level++;
+        round ^= 1;
+        cnt++;
     }
+    write_levels();
+    PTG_CUDA_TRY(cudaGetLastError());
 }
 
 template <class OffT>
@@ -677,7 +755,9 @@ void mssssp_impl(ptg_graph *g, const uint32_t *h_srcs, uint32_t k, uint32_t *d_r
     const uint32_t *col = g->d_col.as<uint32_t>();
     const uint32_t *wt = g->d_w.as<uint32_t>();
     uint32_t base = (flags & PTG_LEVEL_ZERO_BASED) ? 0u : 1u;
-    ms_prepare<OffT>(g, n * 8);
+    ms_prepare<OffT>(g);
+    ws.ms[0].ensure(n * 8);
+    ws.ms[1].ensure(n * 8);
     u64 *M0 = ws.ms[0].as<u64>(), *M1 = ws.ms[1].as<u64>();
     unsigned long long *bsum = ws.bsum.as<unsigned long long>();
     uint32_t *d_srcs = reinterpret_cast<uint32_t *>(bsum + 1024);
@@ -745,25 +825,17 @@ bool ms_group(ptg_graph *g, const uint32_t *h_srcs, uint32_t k, uint32_t *d_rows
         if (o64) mssssp_impl<unsigned long long>(g, h_srcs, k, d_rows, flags, rr);
         else mssssp_impl<uint32_t>(g, h_srcs, k, d_rows, flags, rr);
     } else {
-        // levels are written as vertices are reached, in the stored vertex
-        // order (coalesced; writing by caller id there measured 1.6x slower),
-        // and mapped to caller ids after on a degree-grouped graph
-        uint32_t *rows = d_rows;
-        if (g->relabeled) {
-            g->ctx->ws.relab[1].ensure((uint64_t)k * g->n * 4);
-            rows = g->ctx->ws.relab[1].as<uint32_t>();
-        }
-        if (k <= 64) {
-            if (o64) msbfs_impl<unsigned long long, 1>(g, h_srcs, k, rows, flags, rr);
-            else msbfs_impl<uint32_t, 1>(g, h_srcs, k, rows, flags, rr);
+        // levels go to the rows once, by caller id, from the kept masks
+                if (k <= 64) {
+            if (o64) msbfs_impl<unsigned long long, 1>(g, h_srcs, k, d_rows, flags, rr);
+            else msbfs_impl<uint32_t, 1>(g, h_srcs, k, d_rows, flags, rr);
         } else if (k <= 128) {
-            if (o64) msbfs_impl<unsigned long long, 2>(g, h_srcs, k, rows, flags, rr);
-            else msbfs_impl<uint32_t, 2>(g, h_srcs, k, rows, flags, rr);
+            if (o64) msbfs_impl<unsigned long long, 2>(g, h_srcs, k, d_rows, flags, rr);
+            else msbfs_impl<uint32_t, 2>(g, h_srcs, k, d_rows, flags, rr);
         } else {
-            if (o64) msbfs_impl<unsigned long long, 4>(g, h_srcs, k, rows, flags, rr);
-            else msbfs_impl<uint32_t, 4>(g, h_srcs, k, rows, flags, rr);
+            if (o64) msbfs_impl<unsigned long long, 4>(g, h_srcs, k, d_rows, flags, rr);
+            else msbfs_impl<uint32_t, 4>(g, h_srcs, k, d_rows, flags, rr);
         }
-        if (g->relabeled) unpermute_u32(g, rows, d_rows, k);
     }
     return true;
 }

@@ -248,7 +248,7 @@ struct LevelMsg {
 
 struct Workspace {
     DevBuf value, q[2], bm[2], farbm, vis, scan, rowstart, tiles, bsum, ctl, aux, aux2, flags;
-    DevBuf ms[3];  // multi-source 64-bit masks
+    DevBuf ms[2];  // multi-source 64-bit masks
     DevBuf relab[2];  // results in the stored vertex order, before mapping to caller ids
     PinnedBuf h_ctl, h_flags;
     PinnedBuf h_msg;  // LevelMsg, mapped

@@ -83,15 +83,15 @@ struct Lane {
 
 // Device bytes a lane's workspace needs for a batch of k (an estimate of the
 // buffers the multi-source passes grow).  On a degree-grouped graph the
-// results pass through buffers in the stored order first: the k level rows
-// of a multi-source BFS, one row of the single-source paths.
+// results of the single-source paths pass through a row in the stored order
+// first.
 uint64_t batch_bytes(uint32_t kind, uint64_t n, uint64_t m, uint32_t k, bool regrouped) {
     uint64_t q = 2 * n * 4 + 2 * (n + 1) * 8 + (m / kTile + 4) * 4;
     uint64_t rows = (uint64_t)k * n * 4;
     if (regrouped) q += 2 * n * 4;
     if (kind == PTG_Q_BFS) {
         uint64_t W = k <= 64 ? 1 : (k <= 128 ? 2 : 4);
-        return 3 * n * 8 * W + rows * (regrouped ? 2 : 1) + q;
+        return 13 * n * 8 * W + rows + q;  // 12 levels' masks and the seen mask
     }
     if (kind == PTG_Q_SSSP) return n * 64 * 4 + 2 * n * 8 + rows + q;
     return 2 * n * 32 * 4 + rows + (m / 2048 + 1) * 32 * 8;  // PPR
@@ -99,7 +99,7 @@ uint64_t batch_bytes(uint32_t kind, uint64_t n, uint64_t m, uint32_t k, bool reg
 
 uint64_t ws_bytes(const Workspace &w) {
     const DevBuf *b[] = {&w.value, &w.q[0], &w.q[1], &w.bm[0], &w.bm[1], &w.farbm, &w.vis, &w.scan, &w.rowstart,
-                         &w.tiles, &w.bsum, &w.ctl, &w.aux, &w.aux2, &w.flags, &w.ms[0], &w.ms[1], &w.ms[2],
+                         &w.tiles, &w.bsum, &w.ctl, &w.aux, &w.aux2, &w.flags, &w.ms[0], &w.ms[1],
                          &w.relab[0], &w.relab[1]};
     uint64_t s = 0;
     for (auto *x : b) s += x->bytes;
