@@ -233,10 +233,14 @@ typedef struct ptg_tuning {
                                     unvisited edges / bfs_alpha (default 15)             */
     float bfs_beta;              /* ... and back to push when the frontier holds fewer
                                     than n / bfs_beta vertices (default 18)              */
-    float sssp_delta_scale;      /* default SSSP bucket width = this x the mean edge
-                                    weight on graphs of 2^29+ edges, up to 4x wider on
-                                    smaller ones (default 0.75; 0: label-correcting)     */
-    uint32_t expand_ctas_per_sm; /* push relax (k_expand) CTAs per SM, 1..32 (default 4) */
+    float sssp_delta_scale;      /* default SSSP bucket width of an in-HBM graph = this
+                                    x the mean edge weight x 1/4 on graphs of 2^25+
+                                    edges, up to x 4 on smaller ones; buckets widen as
+                                    a search runs out of edges (default 0.75; 0:
+                                    label-correcting)                                    */
+    uint32_t expand_ctas_per_sm; /* CTAs per SM of the in-HBM traversals and the push
+                                    relax of streamed graphs, 1..32 (default 4; the
+                                    in-HBM kernel takes what fits, at most 4)            */
     uint32_t pr_ctas_per_sm;     /* PageRank SpMV CTAs per SM, 1..32 (default 16)        */
     uint32_t pr_mid;             /* PageRank rows of 5..pr_mid edges run 8 lanes per
                                     row, longer ones a warp (default 256; 8..pr_chunk)   */

@@ -269,8 +269,9 @@ LevelMsg wait_level_msg(Workspace &ws, cudaStream_t st) {
     out.seq = want;
     out.F = __atomic_load_n(&m->F, __ATOMIC_RELAXED);
     out.error = __atomic_load_n(&m->error, __ATOMIC_RELAXED);
-    out.pad = 0;
+    out.pad = __atomic_load_n(&m->pad, __ATOMIC_RELAXED);
     out.frontier_E = __atomic_load_n(&m->frontier_E, __ATOMIC_RELAXED);
+    out.E = __atomic_load_n(&m->E, __ATOMIC_RELAXED);
     return out;
 }
 
@@ -811,21 +812,21 @@ ptg_status run_u32(ptg_graph *g, T *out, uint32_t flags, ptg_run_stats *stats,
             d_out = ctx->ws.value.as<T>();
         }
         RunResult rr;
-        PTG_CUDA_TRY(cudaEventRecord(ctx->ev0, st));
+        // the device time is measured for those who ask for it
+        if (stats) PTG_CUDA_TRY(cudaEventRecord(ctx->ev0, st));
         body(d_out, rr);
-        PTG_CUDA_TRY(cudaEventRecord(ctx->ev1, st));
+        if (stats) PTG_CUDA_TRY(cudaEventRecord(ctx->ev1, st));
         if (!(flags & PTG_OUT_DEVICE))
             PTG_CUDA_TRY(cudaMemcpyAsync(out, d_out, g->n * sizeof(T), cudaMemcpyDeviceToHost, st));
         PTG_CUDA_TRY(cudaStreamSynchronize(st));
         ctx->prof.resolve();
+        if (!stats) return;
         float ms = 0;
         PTG_CUDA_TRY(cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1));
         rr.device_ms = ms;
         fill_stats(stats, rr);
-        if (stats) {
-            stats->vertices_reached = 0;
-            stats->edges_in_component = 0;
-        }
+        stats->vertices_reached = 0;
+        stats->edges_in_component = 0;
     });
 }
 

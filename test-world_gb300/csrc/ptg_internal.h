@@ -126,22 +126,14 @@ struct PinnedBuf {
 struct TravCtl {
     unsigned long long E;         // edges of the current frontier (scan total)
     unsigned long long edges_done;// running total of edges expanded (stats)
-    unsigned long long m_unvisited; // BFS direction heuristic
+    unsigned long long m_unvisited; // multi-source rounds: edges of the new frontier
     unsigned long long far_min;   // min dist over the far pile (near/far SSSP)
-    unsigned long long next_E;    // edges of the next frontier (summed by k_compact for BFS)
     unsigned int F;               // current frontier size
     unsigned int next_tail;       // next frontier append cursor
-    unsigned int far_count;       // far pile size
-    unsigned int far_tail;        // far pile append cursor (split output)
     unsigned int threshold;       // near/far split value (SSSP)
-    unsigned int dir;             // 0 top-down, 1 bottom-up
-    unsigned int level_val;       // BFS: value of current frontier vertices
     unsigned int error;           // nonzero: a kernel detected a bad index
-    unsigned int bu_next;         // bottom-up BFS chunk counter (zero before each round)
-    unsigned int bu_found;        // vertices a bottom-up round reached (its next frontier)
     unsigned int compact_done;    // CTAs of the level's compaction that finished (the last ends the level)
     unsigned int pad;
-    unsigned long long frontier_E;  // unclipped edges of the current frontier (set at the level's end)
 };
 
 // --------------------------------------------------------------------------
@@ -233,22 +225,23 @@ struct Prof {
 // --------------------------------------------------------------------------
 // context / graph
 // --------------------------------------------------------------------------
-// What the host reads at the end of an in-HBM traversal level, written by
-// the last CTA of the level's compaction straight into page-locked host
-// memory (device-mapped) and published by `seq`: the host polls it instead
-// of copying the control block back and synchronizing the stream.
+// What the host reads at the end of an in-HBM traversal or a multi-source
+// round, written by its last thread straight into page-locked host memory
+// (device-mapped) and published by `seq`: the host polls it instead of copying
+// a control block back and synchronizing the stream.
 struct LevelMsg {
     uint32_t seq;    // written last
-    uint32_t F;      // the next frontier's size
-    uint32_t error;  // TravCtl::error
-    uint32_t pad;
-    unsigned long long frontier_E;  // its unclipped edge count (multi-source rounds: unvisited edges)
-    unsigned long long E;           // multi-source rounds: the round's scanned edges
+    uint32_t F;      // rounds: the next frontier's size; traversals: levels run
+    uint32_t error;  // error bits
+    uint32_t pad;    // traversals: pull levels
+    unsigned long long frontier_E;  // rounds: edges of the next frontier
+    unsigned long long E;           // edges scanned
 };
 
 struct Workspace {
     DevBuf value, q[2], bm[2], farbm, vis, scan, rowstart, tiles, bsum, ctl, aux, aux2, flags;
     DevBuf ms[2];  // multi-source 64-bit masks
+    DevBuf res;    // control words of the one-launch traversal (resident.cu)
     DevBuf relab[2];  // results in the stored vertex order, before mapping to caller ids
     PinnedBuf h_ctl, h_flags;
     PinnedBuf h_msg;  // LevelMsg, mapped

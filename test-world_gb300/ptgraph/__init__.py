@@ -446,7 +446,8 @@ class Graph:
         o.flags = flags
         o.delta = delta
         st = RunStats()
-        o.stats = ctypes.pointer(st)
+        if stats is not None:
+            o.stats = ctypes.pointer(st)
         return o, st
 
     def bfs(self, src, flags=0, stats=None, out=None):
@@ -478,7 +479,8 @@ class Graph:
         o = PrOpts()
         o.flags, o.iterations, o.damping = flags, iterations, damping
         st = RunStats()
-        o.stats = ctypes.pointer(st)
+        if stats is not None:
+            o.stats = ctypes.pointer(st)
         _check(lib().ptg_pagerank(self.h, _ptr(out), ctypes.byref(o)), self.ctx.h)
         if stats is not None:
             stats.update(st.as_dict())
@@ -489,7 +491,8 @@ class Graph:
         o = PrOpts()
         o.flags, o.iterations, o.damping = flags, iterations, damping
         st = RunStats()
-        o.stats = ctypes.pointer(st)
+        if stats is not None:
+            o.stats = ctypes.pointer(st)
         _check(lib().ptg_ppr(self.h, src, _ptr(out), ctypes.byref(o)), self.ctx.h)
         if stats is not None:
             stats.update(st.as_dict())
@@ -501,7 +504,8 @@ class Graph:
         o = PrOpts()
         o.flags, o.iterations, o.damping = flags, iterations, damping
         st = RunStats()
-        o.stats = ctypes.pointer(st)
+        if stats is not None:
+            o.stats = ctypes.pointer(st)
         _check(lib().ptg_ppr_batch(self.h, s.ctypes.data_as(_u32p), s.size, _ptr(out), ctypes.byref(o)),
                self.ctx.h)
         if stats is not None:
