@@ -33,11 +33,11 @@ sys.path.insert(0, os.path.join(ROOT, "test-world_gb300"))
 
 PEAKS_FILE = os.path.join(ROOT, "MEASURED_PEAKS.json")
 FALLBACK_HBM_GBS = 6800.0
-# ncu dram__bytes_read.sum + dram__bytes_write.sum of the SpMV kernels of one
-# PageRank iteration (k_pr_small/mid/big/chunks/long) on RMAT scale 22:
-# 584.27 MB + 1.42 MB over n + m = 4,194,304 + 128,307,638 items (built-in tuning:
+# ncu dram__bytes_read.sum + dram__bytes_write.sum of the SpMV kernel of one
+# PageRank iteration (k_pr_iter) on RMAT scale 22:
+# 546.77 MB + 3.52 MB over n + m = 4,194,304 + 128,314,956 items (built-in tuning:
 # degree-grouped vertex order)
-PR_DRAM_BYTES_PER_ITEM = (584.270848e6 + 1.417984e6) / (4194304 + 128307638)
+PR_DRAM_BYTES_PER_ITEM = (546.77e6 + 3.52e6) / (4194304 + 128314956)
 
 
 def make_ctx(args, device):
@@ -816,9 +816,9 @@ def peaks():
 
 def roofline(prof, n, m, step_edges, bfs_edges, args, step_ms):
     """Roofline of the dominant kernel: algorithmic bytes per launch / its average launch time.
-    The PageRank SpMV kernels of one iteration (degree bins, run side by side
-    on forked streams) count as one launch, timed by the library's
-    `pagerank_iteration` span from fork to join; shares are of the step."""
+    A PageRank iteration is one launch (k_pr_iter).  Profiles of several SpMV
+    kernels per iteration (run side by side, or timed as a whole by a
+    `pagerank_iteration` span) count as one launch too; shares are of the step."""
     hbm, kind = peaks()
     span = prof.get("pagerank_iteration")
     agg = {k: v for k, v in prof.items() if k != "pagerank_iteration"}
@@ -827,6 +827,9 @@ def roofline(prof, n, m, step_edges, bfs_edges, args, step_ms):
         for k in pr:
             del agg[k]
         agg["pagerank_spmv"] = span if span else (prof["k_pr_small"][0], sum(prof[k][1] for k in pr))
+    elif "k_pr_iter" in agg:
+        pr = ["k_pr_iter"]
+        agg["pagerank_spmv"] = agg.pop("k_pr_iter")
     top = max(agg.items(), key=lambda kv: kv[1][1])
     name, (cnt, tot) = top
     avg_ms = tot / max(cnt, 1)
@@ -834,7 +837,7 @@ def roofline(prof, n, m, step_edges, bfs_edges, args, step_ms):
     kernels = pr if name == "pagerank_spmv" else [name]
     if name == "pagerank_spmv":
         per_launch = 4 * (n + 1) + 8 * m + 8 * n  # one PageRank iteration
-        unit_desc = "PageRank iteration (k_pr_small/mid/big/chunks/long): 4(n+1) + 8m + 8n bytes"
+        unit_desc = "PageRank iteration (%s): 4(n+1) + 8m + 8n bytes" % "/".join(pr)
         if PR_DRAM_BYTES_PER_ITEM:
             traffic = PR_DRAM_BYTES_PER_ITEM * (n + m)
     else:

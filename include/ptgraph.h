@@ -245,7 +245,9 @@ typedef struct ptg_tuning {
     uint32_t pr_mid;             /* PageRank rows of 5..pr_mid edges run 8 lanes per
                                     row, longer ones a warp (default 256; 8..pr_chunk)   */
     uint32_t pr_chunk;           /* rows over pr_chunk edges are cut into pr_chunk-edge
-                                    pieces (default 4096; 128..65536)                    */
+                                    pieces (default 4096; 128..65536); on graphs under
+                                    2^24 edges both are at most m / 4096 (256 or more)
+                                    and 1/16 of that (32 or more)                        */
     uint32_t ms_pull_small;      /* multi-source pull: rows up to this many edges take
                                     a thread, longer ones warps (default 32; 1..4096)    */
     uint32_t ms_pull_chunk;      /* edges per warp item of a long row (default 1024;

@@ -262,10 +262,6 @@ struct ptg_ctx {
     uint64_t hbm_bytes = 0;
     cudaStream_t stream = nullptr;       // compute stream
     cudaStream_t copy_stream = nullptr;  // host->device partition stream
-    // PageRank degree bins run side by side: streams forked from and joined
-    // back to `stream` every iteration (created on first use)
-    cudaStream_t side[3] = {nullptr, nullptr, nullptr};
-    cudaEvent_t side_fork = nullptr, side_join[3] = {nullptr, nullptr, nullptr};
     bool holds_cache = false;            // counted by the device block cache (devmem.cpp)
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     std::mutex mu;                       // one query at a time per context
@@ -301,8 +297,8 @@ struct ptg_graph {
     uint64_t n_pull_items = 0;
     bool pull_items_built = false;
     uint32_t pull_small = 0, pull_chunk = 0;  // the thresholds the pull items were built with
-    ptg::DevBuf d_pr_mid, d_pr_big, d_pr_items, d_pr_longs;  // PageRank rows binned by degree
-    uint64_t n_pr_mid = 0, n_pr_big = 0, n_pr_items = 0, n_pr_longs = 0;
+    ptg::DevBuf d_pr_mid, d_pr_big, d_pr_items;  // PageRank rows binned by degree
+    uint64_t n_pr_mid = 0, n_pr_big = 0, n_pr_items = 0;
     bool pr_bins_built = false;
     uint32_t pr_mid = 0, pr_chunk = 0;  // the thresholds the bins were built with
     // degree-grouped vertex order (resident symmetric graphs): the arrays

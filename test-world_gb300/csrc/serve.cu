@@ -127,7 +127,6 @@ ptg_graph *make_view(ptg_graph *g, ptg_ctx *lane) {
     alias(v->d_pr_mid, g->d_pr_mid);
     alias(v->d_pr_big, g->d_pr_big);
     alias(v->d_pr_items, g->d_pr_items);
-    alias(v->d_pr_longs, g->d_pr_longs);
     alias(v->d_nzbm, g->d_nzbm);
     alias(v->d_pull_items, g->d_pull_items);
     alias(v->d_perm, g->d_perm);
@@ -142,7 +141,6 @@ ptg_graph *make_view(ptg_graph *g, ptg_ctx *lane) {
     v->n_pr_mid = g->n_pr_mid;
     v->n_pr_big = g->n_pr_big;
     v->n_pr_items = g->n_pr_items;
-    v->n_pr_longs = g->n_pr_longs;
     v->pr_bins_built = g->pr_bins_built;
     v->mean_weight = g->mean_weight;
     v->resident_edges = g->resident_edges;
@@ -164,7 +162,6 @@ void drop_view(ptg_graph *v, const ptg_graph *g) {
     detach(v->d_pr_mid, g->d_pr_mid);
     detach(v->d_pr_big, g->d_pr_big);
     detach(v->d_pr_items, g->d_pr_items);
-    detach(v->d_pr_longs, g->d_pr_longs);
     detach(v->d_nzbm, g->d_nzbm);
     detach(v->d_pull_items, g->d_pull_items);
     detach(v->d_perm, g->d_perm);
