@@ -20,7 +20,9 @@
 //   next mask with one reduction per edge.  Rounds run until no mask is set.
 // Results equal k single-source calls (tests compare them row by row).
 #include <algorithm>
+#include <climits>
 #include <cstring>
+#include <type_traits>
 
 #include "frontier.cuh"
 
@@ -376,6 +378,10 @@ __global__ void k_mss_seed(const uint32_t *srcs, uint32_t k, u64 *A, uint32_t *d
     }
 }
 
+// Bounds of k_mss_queue: none for distances of 2^30 and more.
+constexpr uint32_t kMssFar = 1u << 30;
+constexpr int kMssNone = 0x7F7F7F7F;  // dmax: no bound (any value from here on)
+
 // MS-SSSP round: a warp relaxes one edge at a time for all 64 sources (lane l:
 // sources 2l and 2l+1, one 8-byte load), eight edges per step so eight
 // distance loads per lane are in flight.  Edge slots are tiled like the single-source expand.  The
@@ -383,7 +389,8 @@ __global__ void k_mss_seed(const uint32_t *srcs, uint32_t k, u64 *A, uint32_t *d
 template <class OffT>
 __global__ void __launch_bounds__(kBlock) k_mss_relax(const uint32_t *q, const OffT *sc, const OffT *rs,
                                                       const uint32_t *tr, const uint32_t *col, const uint32_t *w,
-                                                      uint32_t *dist, const u64 *A, u64 *N, const TravCtl *ctl) {
+                                                      uint32_t *dist, const u64 *A, u64 *N, const int *dmin,
+                                                      const int *dmax, const TravCtl *ctl) {
     __shared__ OffT s_sc[kTile + 2];
     __shared__ OffT s_rs[kTile + 2];
     __shared__ uint32_t s_u[kTile + 2];
@@ -436,23 +443,28 @@ __global__ void __launch_bounds__(kBlock) k_mss_relax(const uint32_t *q, const O
                     row_info(r, nx, delta, ul);
                 }
                 uint32_t vl = 0, wl = 0;
+                bool keep = false;
                 if (ok) {
                     uint64_t e = (uint64_t)(OffT)(delta + (OffT)jj);
                     vl = __ldcs(col + e);
                     wl = __ldcs(w + e);
+                    const int top = dmax[vl];  // see k_mss_queue
+                    keep = top >= kMssNone || (long long)dmin[ul] + wl < top;
                 }
                 row = __shfl_sync(0xffffffffu, r, 31);
-                const uint32_t cnt = (uint32_t)min((uint64_t)32, w1 - j);
-                for (uint32_t b = 0; b < cnt; b += 8) {
+                unsigned left = __ballot_sync(0xffffffffu, keep);
+                while (left) {
                     uint32_t vv[8], nd0[8], nd1[8], cur0[8], cur1[8];
 #pragma unroll
                     for (int t = 0; t < 8; t++) {
-                        uint32_t src = (b + t) & 31u;
+                        const bool have = left != 0;
+                        const uint32_t src = have ? __ffs(left) - 1 : 0;
+                        left &= left - 1;
                         uint32_t ut = __shfl_sync(0xffffffffu, ul, src);
                         uint32_t wt = __shfl_sync(0xffffffffu, wl, src);
                         vv[t] = __shfl_sync(0xffffffffu, vl, src);
                         nd0[t] = nd1[t] = PTG_UNREACHED;
-                        if (b + t < cnt) {
+                        if (have) {
                             if (ut != cur_u) {  // warp-uniform: a new tail vertex
                                 cur_u = ut;
                                 am = A[ut];
@@ -486,6 +498,199 @@ __global__ void __launch_bounds__(kBlock) k_mss_relax(const uint32_t *q, const O
         }
         __syncthreads();
     }
+}
+
+// Dense MS-SSSP round on a graph whose edges carry the same weight both ways
+// (graph_weights_symmetric): every vertex takes the least candidate over its
+// neighbours in registers and writes its own distances once.  Pushing the same
+// round sends two reductions of 8 sectors per edge to L2 and takes three times
+// the instructions per edge: 2.4 and 2.1 ms in the two heaviest rounds of 64
+// sources on RMAT-20, 0.9 ms a round on average here.  Work is split as in the MS-BFS pull:
+// rows of up to `small` edges by 32-vertex groups, longer ones in chunks, a
+// warp each; 32 edges are loaded side by side, those that pass the bound of
+// k_mss_queue are taken 8 at a time by the whole warp.  A row in several
+// chunks meets in atomics.  Distances read may be this round's already (they
+// only fall, and an improved vertex is queued for the next round).
+struct MssEdge {
+    uint32_t u, w, lo, hi;  // neighbour, weight, its active sources
+};
+
+template <class OffT>
+__device__ __forceinline__ void mss_pull_row(OffT b, OffT e, uint64_t v, bool alone, const uint32_t *col,
+                                             const uint32_t *w, uint32_t *dist, const u64 *A, u64 *N,
+                                             const int *dmin, int top, MssEdge *pass) {
+    const unsigned lane = lane_id(), bit = 1u << lane;
+    bool loaded = false;
+    uint2 own = make_uint2(0u, 0u), best = own;
+    for (OffT k0 = b; k0 < e; k0 += 32) {
+        const bool ok = k0 + (OffT)lane < e;
+        const uint32_t ul = ok ? __ldcs(col + k0 + lane) : 0u, wl = ok ? __ldcs(w + k0 + lane) : 0u;
+        const u64 al = ok ? A[ul] : 0ull;
+        const bool keep = al != 0 && (top >= kMssNone || (long long)dmin[ul] + wl < top);
+        const unsigned left = __ballot_sync(0xffffffffu, keep);
+        if (!left) continue;
+        // the edges that pass, side by side in shared memory, padded with
+        // edges that no source is active at (reading them back broadcast takes
+        // one instruction where shuffles took nine)
+        const int cnt = __popc(left), at = keep ? __popc(left & lanemask_lt()) : cnt + __popc(~left & lanemask_lt());
+        __syncwarp();
+        pass[at] = MssEdge{keep ? ul : (uint32_t)v, wl, keep ? (uint32_t)al : 0u, keep ? (uint32_t)(al >> 32) : 0u};
+        __syncwarp();
+        if (!loaded) {
+            own = reinterpret_cast<const uint2 *>(dist + v * 64)[lane];
+            best = own;
+            loaded = true;
+        }
+        auto take = [&](auto count, int i) {
+            constexpr int kN = decltype(count)::value;
+            uint2 d[kN];
+#pragma unroll
+            for (int t = 0; t < kN; t++) d[t] = reinterpret_cast<const uint2 *>(dist + (uint64_t)pass[i + t].u * 64)[lane];
+#pragma unroll
+            for (int t = 0; t < kN; t++) {
+                const MssEdge x = pass[i + t];
+                if (x.lo & bit) best.x = min(best.x, d[t].x + x.w);
+                if (x.hi & bit) best.y = min(best.y, d[t].y + x.w);
+            }
+        };
+        int i = 0;
+        for (; i + 4 < cnt; i += 8) take(std::integral_constant<int, 8>{}, i);
+        if (i < cnt) take(std::integral_constant<int, 4>{}, i);
+    }
+    if (!loaded) return;
+    const bool i0 = best.x < own.x, i1 = best.y < own.y;
+    const unsigned b0 = __ballot_sync(0xffffffffu, i0), b1 = __ballot_sync(0xffffffffu, i1);
+    if (!(b0 | b1)) return;
+    if (alone) {
+        reinterpret_cast<uint2 *>(dist + v * 64)[lane] = best;
+        if (lane == 0) N[v] = (u64)b0 | ((u64)b1 << 32);
+    } else {
+        if (i0) atomicMin(&dist[v * 64 + 2 * lane], best.x);
+        if (i1) atomicMin(&dist[v * 64 + 2 * lane + 1], best.y);
+        if (lane == 0) atomicOr(&N[v], (u64)b0 | ((u64)b1 << 32));
+    }
+}
+
+template <class OffT>
+__global__ void __launch_bounds__(kBlock, 5) k_mss_pull(const uint2 *items, uint64_t nitems, uint32_t small,
+                                                     uint32_t chunk, uint64_t n, const OffT *off, const uint32_t *col,
+                                                     const uint32_t *w, uint32_t *dist, const u64 *A, u64 *N,
+                                                     const int *dmin, const int *dmax) {
+    __shared__ __align__(16) MssEdge s_pass[kBlock / 32][32];
+    MssEdge *pass = s_pass[threadIdx.x >> 5];
+    const unsigned lane = lane_id();
+    const uint64_t nwarps = (uint64_t)gridDim.x * (kBlock / 32), wid = (blockIdx.x * (uint64_t)kBlock + threadIdx.x) >> 5;
+    for (uint64_t i = wid; i < nitems; i += nwarps) {
+        const uint2 it = items[i];
+        const OffT row = off[it.x], end = off[(uint64_t)it.x + 1];
+        const OffT b = row + (OffT)it.y * (OffT)chunk;
+        const OffT e = end - b > (OffT)chunk ? b + (OffT)chunk : end;
+        mss_pull_row<OffT>(b, e, it.x, end - row <= (OffT)chunk, col, w, dist, A, N, dmin, dmax[it.x], pass);
+    }
+    for (uint64_t wb = wid; wb * 32 < n; wb += nwarps) {
+        const uint64_t v = wb * 32 + lane;
+        const OffT b = v < n ? off[v] : (OffT)0, e = v < n ? off[v + 1] : (OffT)0;
+        const int top = v < n ? dmax[v] : 0;
+        unsigned rows = __ballot_sync(0xffffffffu, b < e && (uint64_t)(e - b) <= small);
+        while (rows) {
+            const int j = __ffs(rows) - 1;
+            rows &= rows - 1;
+            mss_pull_row<OffT>(__shfl_sync(0xffffffffu, b, j), __shfl_sync(0xffffffffu, e, j), wb * 32 + j, true, col, w,
+                               dist, A, N, dmin, __shfl_sync(0xffffffffu, top, j), pass);
+        }
+    }
+}
+
+// The vertex of the highest degree (the smallest such id).
+template <class OffT>
+__global__ void __launch_bounds__(kBlock) k_mss_hub(const OffT *off, uint64_t n, u64 *best) {
+    u64 b = 0;
+    for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < n; v += (uint64_t)gridDim.x * blockDim.x) {
+        const u64 deg = min((u64)(off[v + 1] - off[v]), 0xffffffffull);
+        b = max(b, deg << 32 | (0xffffffffull - v));
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) b = max(b, __shfl_xor_sync(0xffffffffu, b, o));
+    if (lane_id() == 0) atomicMax(best, b);
+}
+
+// After a round: the queue of the vertices with a new mask, the sum of their
+// degrees (ctl->m_unvisited), the sources that go on (live_next), and per
+// queued vertex the bounds that k_mss_relax drops edges by.  Source s improves
+// v over an edge (u, v) of weight w only if dist[u][s] + w < dist[v][s], with
+// both sides taken less the source's distance to a hub, base[s]: so only if
+// dmin[u] + w < dmax[v], the least such value of u's active sources and the
+// largest of v's live ones.  Less base[s] the sources agree on how far a
+// vertex lies, and the bound lets through little more than improves (RMAT-14,
+// rounds 3 to 7: 69, 25, 12, 7, 5% of the edges, of which 46, 16, 7, 3, 2% improve a
+// source; the plain distances would let 95 ... 63% through).  The sources in
+// `live` are those that had an active vertex a round ago: one whose search has
+// ended, or that never reached this component, does not hold dmax up.  A
+// dmax[v] formed earlier stays a bound, as distances only fall.  With `refresh`
+// (a round over many edges follows) base is brought up to date, and dmax is
+// formed anew for all vertices if that changed it, or if sources have dropped
+// out of live.  Distances of 2^30 and more: no bound.
+template <class OffT>
+__global__ void __launch_bounds__(kBlock) k_mss_queue(const u64 *M, uint64_t n, const OffT *off, uint32_t *q,
+                                                      TravCtl *ctl, const uint32_t *dist, int *dmin, int *dmax,
+                                                      const u64 *hub, const uint32_t *base_was, uint32_t *base,
+                                                      const u64 *was, const u64 *live, u64 *live_next, int refresh) {
+    const unsigned lane = lane_id();
+    const u64 lm = *live;
+    const bool l0 = (lm >> lane) & 1ull, l1 = (lm >> (32 + lane)) & 1ull;
+    // this lane's two sources' distances to the hub, 0 while there is none
+    const uint64_t h = 0xffffffffull - (*hub & 0xffffffffull);
+    uint2 b = reinterpret_cast<const uint2 *>(dist + h * 64)[lane];
+    if (b.x >= kMssFar) b.x = 0;
+    if (b.y >= kMssFar) b.y = 0;
+    const uint2 bw = reinterpret_cast<const uint2 *>(base_was)[lane];
+    if (!refresh) b = bw;
+    const bool all = __any_sync(0xffffffffu, b.x != bw.x || b.y != bw.y) || (refresh && *was != lm);
+    if (blockIdx.x == 0 && threadIdx.x < 32) reinterpret_cast<uint2 *>(base)[lane] = b;
+    unsigned long long degsum = 0;
+    u64 on = 0;
+    const uint64_t nwarps = (uint64_t)gridDim.x * (kBlock / 32);
+    for (uint64_t wb = (blockIdx.x * (uint64_t)kBlock + threadIdx.x) >> 5; wb * 32 < n; wb += nwarps) {
+        const uint64_t v = wb * 32 + lane;
+        const u64 m = v < n ? M[v] : 0ull;
+        on |= m;
+        if (m) {
+            degsum += (unsigned long long)(off[v + 1] - off[v]);
+            warp_append(q, &ctl->next_tail, (unsigned)n, &ctl->error, (uint32_t)v);
+        }
+        __syncwarp();
+        unsigned todo = all ? __ballot_sync(0xffffffffu, v < n) : __ballot_sync(0xffffffffu, m != 0);
+        while (todo) {  // four vertices' distances in flight, the warp's lanes across the sources
+            uint32_t at[4];
+            uint2 d[4];
+#pragma unroll
+            for (int t = 0; t < 4; t++) {
+                at[t] = todo ? __ffs(todo) - 1 : 32u;
+                todo &= todo - 1;
+                d[t] = make_uint2(0u, 0u);
+                if (at[t] < 32) d[t] = reinterpret_cast<const uint2 *>(dist + (wb * 32 + at[t]) * 64)[lane];
+            }
+#pragma unroll
+            for (int t = 0; t < 4; t++) {
+                if (at[t] >= 32) break;
+                const u64 am = __shfl_sync(0xffffffffu, m, at[t]);
+                const bool a0 = (am >> lane) & 1ull, a1 = (am >> (32 + lane)) & 1ull;
+                const bool far0 = d[t].x >= kMssFar, far1 = d[t].y >= kMssFar;
+                const int x0 = (int)d[t].x - (int)b.x, x1 = (int)d[t].y - (int)b.y;  // below 2^30 either way unless far
+                const int lo = min(a0 ? (far0 ? INT_MIN : x0) : INT_MAX, a1 ? (far1 ? INT_MIN : x1) : INT_MAX);
+                const int hi = max(l0 ? (far0 ? kMssNone : x0) : INT_MIN, l1 ? (far1 ? kMssNone : x1) : INT_MIN);
+                const int mn = __reduce_min_sync(0xffffffffu, lo), mx = __reduce_max_sync(0xffffffffu, hi);
+                if (lane == 0) {
+                    if (am) dmin[wb * 32 + at[t]] = mn;
+                    dmax[wb * 32 + at[t]] = mx;
+                }
+            }
+        }
+    }
+    u64 x[1] = {on};
+    live_or<1>(live_next, x);
+    degsum = block_reduce_sum(degsum);
+    if (threadIdx.x == 0 && degsum) atomicAdd(&ctl->m_unvisited, degsum);
 }
 
 // dist[x*64 + s] -> out[s*n + v] for s < k (32 vertices x 64 sources per
@@ -542,6 +747,10 @@ void ms_scan(ptg_ctx *ctx, Workspace &ws, const OffT *off, uint64_t m, uint64_t 
            ws.tiles.as<uint32_t>());
 }
 
+// ws.bsum: scan partials | 256 sources | MS-BFS: all-sources mask, two
+// live-source masks; MS-SSSP: four live-source words, the hub, two bases
+constexpr uint64_t kMsSmall = 1024 * 8 + 256 * 4 + 5 * 8 + 2 * 64 * 4;
+
 template <class OffT>
 void ms_prepare(ptg_graph *g) {
     Workspace &ws = g->ctx->ws;
@@ -551,8 +760,7 @@ void ms_prepare(ptg_graph *g) {
     ws.scan.ensure((n + 1) * sizeof(OffT));
     ws.rowstart.ensure((n + 1) * sizeof(OffT));
     ws.tiles.ensure((m / kTile + 4) * 4);
-    // scan partials | 256 sources | all-sources mask | two live-source masks
-    ws.bsum.ensure(1024 * 8 + 256 * 4 + 3 * 32);
+    ws.bsum.ensure(kMsSmall);
     ws.ctl.ensure(sizeof(TravCtl));
     ws.h_ctl.ensure(sizeof(TravCtl));
     ensure_level_msg(ws);
@@ -762,8 +970,9 @@ void mssssp_impl(ptg_graph *g, const uint32_t *h_srcs, uint32_t k, uint32_t *d_r
     unsigned long long *bsum = ws.bsum.as<unsigned long long>();
     uint32_t *d_srcs = reinterpret_cast<uint32_t *>(bsum + 1024);
     TravCtl *d_ctl = ws.ctl.as<TravCtl>();
-    ws.aux.ensure(n * 64 * 4);
+    ws.aux.ensure(n * 64 * 4 + 2 * n * 4);
     uint32_t *dist = ws.aux.as<uint32_t>();
+    int *dmin = reinterpret_cast<int *>(dist + n * 64), *dmax = dmin + n;
     PTG_CUDA_TRY(cudaMemsetAsync(dist, 0xFF, n * 64 * 4, st));
     PTG_CUDA_TRY(cudaMemsetAsync(M0, 0, n * 8, st));
     PTG_CUDA_TRY(cudaMemsetAsync(M1, 0, n * 8, st));
@@ -773,8 +982,30 @@ void mssssp_impl(ptg_graph *g, const uint32_t *h_srcs, uint32_t k, uint32_t *d_r
     TravCtl init{};
     PTG_CUDA_TRY(cudaMemcpyAsync(d_ctl, &init, sizeof(TravCtl), cudaMemcpyHostToDevice, st));
     int vgrid = grid_for(n, kBlock, sms * 8);
-    launch(ctx, "k_msb_queue", k_msb_queue<OffT, 1>, vgrid, kBlock, 0, st, (const u64 *)M0, n, off,
-           ws.q[1].as<uint32_t>(), d_ctl);
+    // live sources of the last rounds, four words used in turn: two read, one
+    // written, one cleared for the next round
+    u64 *d_live = reinterpret_cast<u64 *>(d_srcs + 256);
+    PTG_CUDA_TRY(cudaMemsetAsync(d_live, 0xFF, 16, st));
+    PTG_CUDA_TRY(cudaMemsetAsync(d_live + 2, 0, 16, st));
+    const bool can_pull = graph_weights_symmetric(g);
+    if (can_pull && !g->pull_items_built) build_pull_items<OffT>(g);
+    // the hub, and the sources' distances to it as of the last two rounds
+    u64 *d_hub = d_live + 4;
+    uint32_t *d_base = reinterpret_cast<uint32_t *>(d_hub + 1);
+    PTG_CUDA_TRY(cudaMemsetAsync(d_hub, 0, 8, st));
+    PTG_CUDA_TRY(cudaMemsetAsync(d_base, 0, 64 * 4, st));
+    PTG_CUDA_TRY(cudaMemsetAsync(dmax, 0x7F, n * 4, st));  // kMssNone
+    launch(ctx, "k_mss_hub", k_mss_hub<OffT>, vgrid, kBlock, 0, st, off, n, d_hub);
+    uint32_t round = 0;
+    auto queue = [&](const u64 *M, bool refresh) {
+        launch(ctx, "k_mss_queue", k_mss_queue<OffT>, vgrid, kBlock, 0, st, M, n, off, ws.q[1].as<uint32_t>(), d_ctl,
+               (const uint32_t *)dist, dmin, dmax, (const u64 *)d_hub, (const uint32_t *)d_base + round % 2 * 64,
+               d_base + (round + 1) % 2 * 64, (const u64 *)d_live + round % 4,
+               (const u64 *)d_live + (round + 1) % 4, d_live + (round + 2) % 4, refresh ? 1 : 0);
+        PTG_CUDA_TRY(cudaMemsetAsync(d_live + round % 4, 0, 8, st));
+        round++;
+    };
+    queue(M0, false);
     uint64_t F, Eact, E;
     ms_next(ctx, ws, F, Eact, E);
     int cur = 0;
@@ -783,22 +1014,29 @@ void mssssp_impl(ptg_graph *g, const uint32_t *h_srcs, uint32_t k, uint32_t *d_r
         if (rr.iterations >= max_rounds) throw Error{PTG_ERR_TIMEOUT, "iteration limit reached"};
         rr.iterations++;
         u64 *Mc = cur ? M1 : M0, *Mn = cur ? M0 : M1;
-        ms_scan<OffT>(ctx, ws, off, m, F, d_ctl);
         PTG_CUDA_TRY(cudaMemsetAsync(Mn, 0, n * 8, st));
-        launch(ctx, "k_mss_relax", k_mss_relax<OffT>, sms * 6, kBlock, 0, st, (const uint32_t *)ws.q[0].p,
-               (const OffT *)ws.scan.p, (const OffT *)ws.rowstart.p, (const uint32_t *)ws.tiles.p, col, wt, dist,
-               (const u64 *)Mc, Mn, (const TravCtl *)d_ctl);
-        launch(ctx, "k_msb_queue", k_msb_queue<OffT, 1>, vgrid, kBlock, 0, st, (const u64 *)Mn, n, off,
-               ws.q[1].as<uint32_t>(), d_ctl);
+        const bool pull = can_pull && Eact * 2 > m;
+        const uint64_t scanned = Eact;
+        if (pull) {
+            launch(ctx, "k_mss_pull", k_mss_pull<OffT>, sms * 8, kBlock, 0, st, (const uint2 *)g->d_pull_items.p,
+                   g->n_pull_items, g->pull_small, g->pull_chunk, n, off, col, wt, dist, (const u64 *)Mc, Mn,
+                   (const int *)dmin, (const int *)dmax);
+        } else {
+            ms_scan<OffT>(ctx, ws, off, m, F, d_ctl);
+            launch(ctx, "k_mss_relax", k_mss_relax<OffT>, sms * 6, kBlock, 0, st, (const uint32_t *)ws.q[0].p,
+                   (const OffT *)ws.scan.p, (const OffT *)ws.rowstart.p, (const uint32_t *)ws.tiles.p, col, wt, dist,
+                   (const u64 *)Mc, Mn, (const int *)dmin, (const int *)dmax, (const TravCtl *)d_ctl);
+        }
+        // a refresh reads every distance, which a round over a large part of the edges repays
+        queue(Mn, Eact * 8 > m);
         PTG_CUDA_TRY(cudaGetLastError());
         ms_next(ctx, ws, F, Eact, E);
-        rr.edges_relaxed += E;
+        rr.edges_relaxed += pull ? scanned : E;
         cur ^= 1;
     }
     launch(ctx, "k_mss_transpose", k_mss_transpose, grid_for((n + 31) / 32, 1, sms * 8), kBlock, 0, st,
            (const uint32_t *)dist, n, k, (const uint32_t *)(g->relabeled ? g->d_newid.p : nullptr), d_rows);
     PTG_CUDA_TRY(cudaGetLastError());
-    (void)Eact;
 }
 
 }  // namespace
@@ -806,8 +1044,10 @@ void mssssp_impl(ptg_graph *g, const uint32_t *h_srcs, uint32_t k, uint32_t *d_r
 // Builds the per-graph tables of the fused passes (pull work items) now
 // rather than on first use.
 void ms_prepare_graph(ptg_graph *g) {
-    if (g->out_of_core || !g->symmetric || g->pull_items_built) return;
-    g->ctx->ws.bsum.ensure(1024 * 8 + 256 * 4 + 3 * 32);
+    if (g->out_of_core || !g->symmetric) return;
+    graph_weights_symmetric(g);
+    if (g->pull_items_built) return;
+    g->ctx->ws.bsum.ensure(kMsSmall);
     if (g->off64) build_pull_items<unsigned long long>(g);
     else build_pull_items<uint32_t>(g);
 }

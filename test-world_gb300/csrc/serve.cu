@@ -93,7 +93,7 @@ uint64_t batch_bytes(uint32_t kind, uint64_t n, uint64_t m, uint32_t k, bool reg
         uint64_t W = k <= 64 ? 1 : (k <= 128 ? 2 : 4);
         return 13 * n * 8 * W + rows + q;  // 12 levels' masks and the seen mask
     }
-    if (kind == PTG_Q_SSSP) return n * 64 * 4 + 2 * n * 8 + rows + q;
+    if (kind == PTG_Q_SSSP) return n * 66 * 4 + 2 * n * 8 + rows + q;
     return 2 * n * 32 * 4 + rows + (m / 2048 + 1) * 32 * 8;  // PPR
 }
 
@@ -143,6 +143,7 @@ ptg_graph *make_view(ptg_graph *g, ptg_ctx *lane) {
     v->n_pr_items = g->n_pr_items;
     v->pr_bins_built = g->pr_bins_built;
     v->mean_weight = g->mean_weight;
+    v->weights_symmetric = g->weights_symmetric;
     v->resident_edges = g->resident_edges;
     v->device_bytes = 0;
     return v;

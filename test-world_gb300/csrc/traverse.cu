@@ -455,6 +455,45 @@ __global__ void __launch_bounds__(kBlock) k_relax_partition(uint64_t e_begin, ui
     }
 }
 
+// Sum over the edges u < v of a hash of (u, v, w), less the same over the
+// edges u > v: zero when the two lists of (smaller end, larger end, weight) are
+// the same (and, where they differ, with probability 2^-64).  Edge-centric
+// tiles; a thread walks the rows of its 8 consecutive edges in registers.
+template <class OffT>
+__global__ void __launch_bounds__(kBlock) k_weight_balance(uint64_t m, uint64_t n, const OffT *off, const uint32_t *col,
+                                                           const uint32_t *w, unsigned long long *out) {
+    __shared__ OffT s_off[kTile + 2];
+    unsigned long long sum = 0;
+    const uint64_t ntiles = (m + kTile - 1) / kTile;
+    for (uint64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+        const uint64_t t0 = tile * kTile, t1 = min(m, t0 + kTile);
+        const uint64_t r0 = block_last_le(off, 0, n, t0), r1 = block_last_le(off, r0, n, t1 - 1);
+        const uint64_t nrows = r1 - r0 + 1;
+        const bool staged = nrows <= (uint64_t)kTile;
+        if (staged)
+            for (uint64_t k = threadIdx.x; k <= nrows; k += kBlock) s_off[k] = off[r0 + k];
+        __syncthreads();
+        const uint64_t j0 = t0 + threadIdx.x * (kTile / kBlock);
+        uint64_t row = 0;
+        if (j0 < t1) row = staged ? last_le(s_off, 0, nrows, j0) : last_le(off, r0, r0 + nrows, j0) - r0;
+        for (int i = 0; i < kTile / kBlock; i++) {
+            const uint64_t j = j0 + i;
+            if (j >= t1) break;
+            while (j >= (uint64_t)(staged ? s_off[row + 1] : off[r0 + row + 1])) row++;
+            const unsigned long long u = r0 + row, v = col[j];
+            unsigned long long h = (min(u, v) << 32 | max(u, v)) * 0x9E3779B97F4A7C15ull;
+            h = (h ^ (h >> 29) ^ ((unsigned long long)w[j] << 20)) * 0xBF58476D1CE4E5B9ull;
+            h = (h ^ (h >> 32) ^ w[j]) * 0x94D049BB133111EBull;
+            h ^= h >> 31;
+            if (u < v) sum += h;
+            if (u > v) sum -= h;
+        }
+        __syncthreads();
+    }
+    sum = block_reduce_sum(sum);
+    if (threadIdx.x == 0 && sum) atomicAdd(out, sum);
+}
+
 // Near/far: smallest distance in the far pile (a bitmap).
 __global__ void __launch_bounds__(kBlock) k_far_min(const uint32_t *far_bm, uint64_t words,
                                                     const uint32_t *value, TravCtl *ctl) {
@@ -822,6 +861,30 @@ void trav_prepare_graph(ptg_graph *g) {
     if (g->out_of_core) return;
     if (g->symmetric) build_nonzero_bits(g);
     measure_mean_weight(g);
+}
+
+bool graph_weights_symmetric(ptg_graph *g) {
+    if (g->weights_symmetric < 0) {
+        g->weights_symmetric = 0;
+        if (g->symmetric && g->weighted && !g->out_of_core && g->m) {
+            ptg_ctx *ctx = g->ctx;
+            cudaStream_t st = ctx->stream;
+            ctx->ws.bsum.ensure(1024 * 8);
+            unsigned long long *acc = ctx->ws.bsum.as<unsigned long long>(), sum = 0;
+            PTG_CUDA_TRY(cudaMemsetAsync(acc, 0, 8, st));
+            const int grid = grid_for(g->m, kTile, ctx->sm_count * 8);
+            if (g->off64)
+                launch(ctx, "k_weight_balance", k_weight_balance<unsigned long long>, grid, kBlock, 0, st, g->m, g->n,
+                       g->d_off.as<unsigned long long>(), g->d_col.as<uint32_t>(), g->d_w.as<uint32_t>(), acc);
+            else
+                launch(ctx, "k_weight_balance", k_weight_balance<uint32_t>, grid, kBlock, 0, st, g->m, g->n,
+                       g->d_off.as<uint32_t>(), g->d_col.as<uint32_t>(), g->d_w.as<uint32_t>(), acc);
+            PTG_CUDA_TRY(cudaMemcpyAsync(&sum, acc, 8, cudaMemcpyDeviceToHost, st));
+            PTG_CUDA_TRY(cudaStreamSynchronize(st));
+            g->weights_symmetric = sum == 0;
+        }
+    }
+    return g->weights_symmetric == 1;
 }
 
 double graph_mean_weight(ptg_graph *g) {

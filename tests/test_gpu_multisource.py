@@ -43,3 +43,30 @@ def test_levels_kept_and_written(ptg, ctx, ctx_grouped, oracle, grouped, wide, l
         assert (rows[i] == known[s][0]).all()
         assert (dist[i] == known[s][1]).all()
     G.close()
+
+
+@pytest.mark.parametrize("grouped", [False, True])
+@pytest.mark.parametrize("both_ways", [True, False])
+@pytest.mark.parametrize("n,m,k", [(300, 4000, 64), (2001, 9000, 5), (5000, 400000, 64)])
+def test_dense_sssp_rounds(ptg, ctx, ctx_grouped, oracle, grouped, both_ways, n, m, k):
+    """Rounds over most of the edges, with the same weight both ways (they may
+    be pulled) and with a weight of its own on every directed edge (they may
+    not), rows around the pull split, a second component and large weights."""
+    rng = np.random.RandomState(n)
+    a, b = rng.randint(0, n - 40, m), (rng.randint(0, n - 40, m) * rng.randint(0, 2, m)) // 2
+    a, b = np.concatenate([a, np.full(33, n - 1)]), np.concatenate([b, n - 2 - np.arange(33)])
+    keep = a != b
+    a, b = a[keep], b[keep]
+    key = np.unique(np.concatenate([a, b]).astype(np.int64) * n + np.concatenate([b, a]))
+    off = np.zeros(n + 1, np.uint64)
+    off[1:] = np.cumsum(np.bincount(key // n, minlength=n))
+    row, col = key // n, key % n
+    mix = np.minimum(row, col) * 7919 + np.maximum(row, col) * 31 if both_ways else row * 7919 + col * 31
+    w = np.where(mix % 97 == 0, 1 << 29, mix % 64).astype(np.uint32)
+    G = (ctx_grouped if grouped else ctx).graph(off, col.astype(np.uint32), w, symmetric=True)
+    srcs = rng.randint(0, n, k).astype(np.uint32)
+    srcs[0] = n - 1
+    dist = G.mssssp(srcs)
+    for i, s in enumerate(srcs):
+        assert (dist[i] == oracle.sssp(off, col.astype(np.uint32), w, int(s))).all()
+    G.close()
