@@ -293,6 +293,7 @@ struct ptg_graph {
     ptg::DevBuf d_off, d_col, d_w, d_invdeg;
     ptg::DevBuf d_nzbm;   // bitmap of vertices with edges (bottom-up BFS), built on first use
     double mean_weight = 0;  // mean resident edge weight (SSSP bucket width), measured on first use
+    uint32_t min_weight = 0;  // least resident edge weight (measured with it)
     int weights_symmetric = -1;  // every edge carries the same weight both ways (checked on first use; -1: not yet)
     ptg::DevBuf d_pull_items;  // (vertex, chunk) work items of high-degree vertices (multi-source pull)
     uint64_t n_pull_items = 0;
@@ -360,11 +361,12 @@ enum TravKind { TRAV_BFS = 0, TRAV_SSSP = 1, TRAV_CCPROP = 2 };
 
 void run_traversal(ptg_graph *g, TravKind kind, uint32_t src, uint32_t *d_value, uint32_t flags,
                    uint32_t delta, uint32_t max_iters, RunResult &rr);
-// Mean resident edge weight of a weighted graph (measured once per graph).
-double graph_mean_weight(ptg_graph *g);
 // Whether a resident weighted graph has, for every edge u->v, an edge v->u of the
 // same weight (checked once per graph; false without PTG_CSR_SYMMETRIC).
 bool graph_weights_symmetric(ptg_graph *g);
+// An SSSP round over fewer edges than this always pushes (40 us of them: a pull
+// round's count, lists and barriers take about as long).
+constexpr uint64_t kSsspPullEdges = 1ull << 23;
 void run_cc_hook(ptg_graph *g, uint32_t *d_label, RunResult &rr);
 void run_pagerank(ptg_graph *g, bool personalized, uint32_t src, double damping, uint32_t iters,
                   float *d_rank, RunResult &rr);

@@ -28,8 +28,14 @@
 //  * BFS pull rounds (each unvisited vertex looks for a parent in the frontier
 //    bitmap) when the frontier's edges outweigh the unvisited ones (Beamer).
 //  * SSSP parks vertices at or above the threshold in a bitmap; when the near
-//    frontier is empty the threshold moves past the smallest parked distance.
-//    Buckets whose edges cost less than the bucket itself double the width.
+//    frontier is empty one pass over them takes those below the next threshold
+//    and finds the smallest distance above it, from which an empty bucket goes
+//    on.  Buckets whose edges cost less than the bucket itself double the
+//    width.
+//  * A heavy SSSP round pulls when the edges carry the same weight both ways:
+//    only vertices above the frontier's least distance plus the least weight
+//    can still improve, on RMAT-24 with 119 M edges in the round whose
+//    frontier has 307 M.
 //
 // Phases hand data over through global memory across the grid barrier (its
 // acquire makes earlier phases' stores visible to ordinary loads).  Within a
@@ -39,10 +45,10 @@
 //
 // What bounds it: a small graph's level is a chain of dependent reads and the
 // barrier, 5-10 us; the heavy SSSP rounds of RMAT-24 probe 190-290 G targets/s,
-// about what PageRank's gathers reach from L2 (one 32-byte sector each).
-// Staging the edges ahead with cp.async and dropping candidates by the largest
+// about what PageRank's gathers reach from L2 (one 32-byte sector each): the
+// round of 307 M edges took 1170 us as a push and takes 730 as a pull.  Staging the edges ahead with cp.async and dropping candidates by the largest
 // distance among the hubs changed neither.  Per search, before -> now: BFS on
-// RMAT-16 217 -> 87 us, on RMAT-24 580 -> 415 us; SSSP on RMAT-24 6.7 -> 4.8
+// RMAT-16 217 -> 87 us, on RMAT-24 580 -> 415 us; SSSP on RMAT-24 6.7 -> 3.5
 // ms; a served mix of small graphs 8.8 -> 6.5 ms.
 #include <algorithm>
 #include <cmath>
@@ -78,9 +84,13 @@ struct ResCtl {
     // kSmallDeg, and longer ones << 32 | their pieces
     u64 few[3], items[3], bigs[3];
     u64 found[3], edges[3];         // the frontier's vertices and edges
-    u64 far_min[2];
+    u64 far_min[3];                 // SSSP: least distance that stays parked, by turn
     u64 cands[4];                   // unvisited vertices that a pull round looked at (level % 4)
     unsigned chunk[2];              // pull work counter, by level parity
+    // SSSP: least distance of the frontier (slot level % 3); edges that a pull
+    // round would look at and its lists (items, bigs), by turn
+    unsigned least[3];
+    u64 pull_edges[2], pull_items[2], pull_bigs[2];
     LevelMsg msg;                   // the outcome, where host memory cannot be mapped
 };
 
@@ -99,6 +109,8 @@ struct ResArgs {
     uint32_t src, base, delta, max_iters;
     float alpha, beta;
     int use_far;
+    int can_pull;                   // SSSP: the same weight both ways on every edge
+    uint32_t min_weight;
     ResCtl *ctl;
     LevelMsg *msg;                  // where the outcome goes (host-mapped, or ctl->msg)
     uint32_t seq;
@@ -150,6 +162,7 @@ __device__ bool grid_barrier(ResCtl *c) {
 struct WarpBuf {
     uint32_t *v;
     uint32_t cnt;
+    uint32_t least;  // SSSP: least improved distance below the threshold
     u64 found, edges;
 };
 
@@ -158,11 +171,12 @@ struct Frontier {
     uint32_t *few, *q;
     uint2 *big;
     u64 *nfew, *items, *bigs;
+    unsigned *least;  // (may be null)
 };
 
 __device__ __forceinline__ Frontier frontier_of(const ResArgs &a, int buf, int slot) {
     return Frontier{a.few[buf],          a.q[buf],   a.big[buf], &a.ctl->few[slot], &a.ctl->items[slot],
-                    &a.ctl->bigs[slot]};
+                    &a.ctl->bigs[slot], &a.ctl->least[slot]};
 }
 
 // The last min(64, cnt) buffered vertices go to the frontier's lists: their
@@ -256,6 +270,11 @@ __device__ __forceinline__ void buf_finish(WarpBuf &b, const ResArgs &a, const F
     while (b.cnt) buf_flush<OffT>(b, a, f);
     if (found) buf_total(b, found, edges);
     else b.found = b.edges = 0;  // counted before
+    if (f.least) {
+        const uint32_t least = __reduce_min_sync(0xffffffffu, b.least);
+        if (lane_id() == 0 && least != PTG_UNREACHED) atomicMin(f.least, least);
+        b.least = PTG_UNREACHED;
+    }
 }
 
 // Calls f(i, word of lane i) for the non-zero words of a warp's 32, all lanes
@@ -324,6 +343,7 @@ __device__ __forceinline__ void relax_edges(const ResArgs &a, const uint32_t (&v
         for (int i = 0; i < U; i++) {
             claim[i] = nd[i] < cur[i];
             if (claim[i]) atomicMin(&a.value[v[i]], nd[i]);
+            if (MODE == 1 && claim[i] && nd[i] < thr) b.least = min(b.least, nd[i]);
         }
         uint32_t old[U];
 #pragma unroll
@@ -450,6 +470,111 @@ __device__ void push_phase(const ResArgs &a, const Frontier &f, uint32_t level_v
     buf_finish<OffT>(b, a, nx, found, edges);
 }
 
+// SSSP pull (symmetric graphs with the same weight both ways): candidates for
+// a vertex over K edges of its row.  Any end below the threshold may give one:
+// what is not in the frontier was relaxed before and improves nothing, and
+// asking the frontier's bitmap first would be one more random read per edge
+// (1060 us instead of 440 for 119 M edges, of which 6.3 M vertices with up to
+// kFewDeg edges took 8 lanes each).
+template <class OffT, int K>
+__device__ __forceinline__ uint32_t pull_edges(const ResArgs &a, OffT begin, uint32_t len, uint32_t o, uint32_t step,
+                                               uint32_t thr, u64 pol) {
+    uint32_t c[K], w[K], best = PTG_UNREACHED;
+#pragma unroll
+    for (int i = 0; i < K; i++) {
+        const bool ok = o + step * i < len;
+        c[i] = ok ? ld_edge(a.col + begin + o + step * i, pol) : PTG_UNREACHED;
+        w[i] = ok ? ld_edge(a.w + begin + o + step * i, pol) : 0u;
+    }
+#pragma unroll
+    for (int i = 0; i < K; i++) c[i] = c[i] != PTG_UNREACHED ? a.value[c[i]] : PTG_UNREACHED;
+#pragma unroll
+    for (int i = 0; i < K; i++)
+        if (c[i] < thr) best = min(best, c[i] + w[i]);
+    return best;
+}
+
+// Vertices above `above` with up to kFewDeg edges, a lane each (the rows of a
+// warp's neighbouring vertices are one run of memory, and grouped by degree
+// they are equally long); longer ones are listed in `look`.
+template <class OffT>
+__device__ void sssp_pull_few(const ResArgs &a, uint32_t above, uint32_t thr, uint32_t *bm_next, const Frontier &nx,
+                              WarpBuf &b, const Frontier &look, WarpBuf &longer) {
+    const OffT *off = reinterpret_cast<const OffT *>(a.off);
+    const uint64_t nthreads = (uint64_t)gridDim.x * kBlock;
+    const u64 pol = l2_evict_first_policy();
+    for (uint64_t v0 = ((uint64_t)blockIdx.x * kBlock + threadIdx.x) & ~31ull; v0 < a.n; v0 += nthreads) {
+        const uint64_t v = v0 + lane_id();
+        OffT begin = 0;
+        uint32_t len = 0;
+        if (v < a.n && a.value[v] > above) {
+            begin = off[v];
+            len = (uint32_t)(off[v + 1] - begin);
+        }
+        buf_add(longer, len > kFewDeg, (uint32_t)v);
+        while (longer.cnt >= 64) buf_flush<OffT>(longer, a, look);
+        if (len > kFewDeg) len = 0;
+        const uint32_t most = __reduce_max_sync(0xffffffffu, len);
+        if (!most) continue;
+        uint32_t best = PTG_UNREACHED;
+        for (uint32_t o = 0; o < most; o += 4) best = min(best, pull_edges<OffT, 4>(a, begin, len, o, 1, thr, pol));
+        const uint32_t t[1] = {best != PTG_UNREACHED ? (uint32_t)v : PTG_UNREACHED}, nd[1] = {best};
+        relax_edges<OffT, 1, 1>(a, t, nd, thr, bm_next, nx, b);
+    }
+    buf_finish<OffT>(longer, a, look, nullptr, nullptr);
+}
+
+// The longer ones: 8 lanes each up to kSmallDeg edges, else a warp per piece
+// (an equal run of pieces per warp, as in push_phase).
+template <class OffT>
+__device__ void sssp_pull_longer(const ResArgs &a, const Frontier &look, uint32_t thr, uint32_t *bm_next,
+                                 const Frontier &nx, WarpBuf &b, u64 *found, u64 *edges) {
+    const OffT *off = reinterpret_cast<const OffT *>(a.off);
+    const unsigned lane = lane_id(), sub = lane & 7u;
+    const u64 warps = (u64)gridDim.x * kWarps, warp = (u64)blockIdx.x * kWarps + (threadIdx.x >> 5);
+    const u64 pol = l2_evict_first_policy();
+    const u64 bigs = *look.bigs, pieces = bigs & 0xffffffffull, count = bigs >> 32;
+    u64 p = pieces * warp / warps;
+    const u64 p1 = pieces * (warp + 1) / warps;
+    if (p < p1) {
+        u64 at = 0, hi = count;  // last entry with at most p pieces before it
+        while (hi - at > 1) {
+            const u64 mid = (at + hi) >> 1;
+            if (look.big[mid].y <= p) at = mid;
+            else hi = mid;
+        }
+        for (; p < p1 && at < count; at++) {
+            const uint2 e = look.big[at];
+            const OffT row = off[e.x], deg = off[(uint64_t)e.x + 1] - row;
+            uint32_t best = PTG_UNREACHED;
+            for (; p < p1; p++) {
+                const u64 k = (p - e.y) * kPiece;
+                if (k >= (u64)deg) break;
+                const uint32_t len = (uint32_t)min((u64)kPiece, (u64)deg - k);
+                best = min(best, pull_edges<OffT, 8>(a, row + (OffT)k, len, lane, 32, thr, pol));
+            }
+            best = __reduce_min_sync(0xffffffffu, best);
+            const uint32_t t[1] = {lane == 0 && best != PTG_UNREACHED ? e.x : PTG_UNREACHED}, nd[1] = {best};
+            relax_edges<OffT, 1, 1>(a, t, nd, thr, bm_next, nx, b);
+        }
+    }
+    const u64 items = *look.items;
+    for (u64 i0 = warp * 4; i0 < items; i0 += warps * 4) {
+        const u64 i = i0 + (lane >> 3);
+        const uint32_t u = i < items ? look.q[i] : 0u;
+        const OffT begin = i < items ? off[u] : (OffT)0;
+        const uint32_t len = i < items ? (uint32_t)(off[(uint64_t)u + 1] - begin) : 0u;
+        const uint32_t most = __reduce_max_sync(0xffffffffu, len);
+        uint32_t best = PTG_UNREACHED;
+        for (uint32_t o = 0; o < most; o += 64) best = min(best, pull_edges<OffT, 8>(a, begin, len, o + sub, 8, thr, pol));
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) best = min(best, __shfl_xor_sync(0xffffffffu, best, o));
+        const uint32_t t[1] = {sub == 0 && best != PTG_UNREACHED ? u : PTG_UNREACHED}, nd[1] = {best};
+        relax_edges<OffT, 1, 1>(a, t, nd, thr, bm_next, nx, b);
+    }
+    buf_finish<OffT>(b, a, nx, found, edges);
+}
+
 // One pull phase of BFS (symmetric graphs): a warp takes `step` bitmap words
 // of vertices, lists the unvisited ones with edges, tests two per lane at a
 // time (offsets, first four neighbours and their frontier bits in flight
@@ -549,7 +674,7 @@ __device__ void pull_phase(const ResArgs &a, const uint32_t *bm_cur, uint32_t *b
         __syncwarp();
     }
     if (lane == 0 && ncands) atomicAdd(cands, ncands);
-    WarpBuf b{nullptr, 0, nfound, nedges};
+    WarpBuf b{nullptr, 0, PTG_UNREACHED, nfound, nedges};
     buf_total(b, found, edges);
 }
 
@@ -558,13 +683,14 @@ __global__ void __launch_bounds__(kBlock, 4) k_traverse(ResArgs a) {
     __shared__ uint32_t s_buf[kWarps][kBuf];
     __shared__ uint32_t s_list[MODE == 0 ? kWarps : 1][MODE == 0 ? kBuWords * 32 : 1];
     __shared__ uint32_t s_mark[MODE == 0 ? kWarps : 1][32];
+    __shared__ uint32_t s_look[MODE == 1 ? kWarps : 1][96];
     const OffT *off = reinterpret_cast<const OffT *>(a.off);
     ResCtl *ctl = a.ctl;
     const unsigned wid = threadIdx.x >> 5;
     const uint64_t tid = (uint64_t)blockIdx.x * kBlock + threadIdx.x, nthreads = (uint64_t)gridDim.x * kBlock;
     const uint64_t words = (a.n + 31) / 32;
     const bool leader = tid == 0;
-    WarpBuf buf{s_buf[wid], 0, 0, 0};
+    WarpBuf buf{s_buf[wid], 0, PTG_UNREACHED, 0, 0};
 
     // ---- initial state ----
     for (uint64_t i = tid; i < a.n; i += nthreads) a.value[i] = MODE == 2 ? (uint32_t)i : PTG_UNREACHED;
@@ -576,9 +702,11 @@ __global__ void __launch_bounds__(kBlock, 4) k_traverse(ResArgs a) {
     }
     if (leader) {
         for (int i = 0; i < 3; i++) ctl->few[i] = ctl->items[i] = ctl->bigs[i] = ctl->found[i] = ctl->edges[i] = 0;
-        ctl->far_min[0] = ctl->far_min[1] = ~0ull;
+        for (int i = 0; i < 3; i++) ctl->far_min[i] = ~0ull;
         ctl->chunk[0] = ctl->chunk[1] = 0;
         for (int i = 0; i < 4; i++) ctl->cands[i] = 0;
+        for (int i = 0; i < 3; i++) ctl->least[i] = PTG_UNREACHED;
+        for (int i = 0; i < 2; i++) ctl->pull_edges[i] = ctl->pull_items[i] = ctl->pull_bigs[i] = 0;
         ctl->error = 0;
     }
     if (!grid_barrier(ctl)) return;
@@ -593,6 +721,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_traverse(ResArgs a) {
                     a.vis[s >> 5] = 1u << (s & 31u);
                     a.bm[0][s >> 5] = 1u << (s & 31u);
                 }
+                ctl->least[0] = a.base;
                 if (deg > kSmallDeg) {
                     a.big[0][0] = make_uint2(s, 0u);
                     ctl->bigs[0] = 1ull << 32 | (deg + kPiece - 1) / kPiece;
@@ -608,11 +737,12 @@ __global__ void __launch_bounds__(kBlock, 4) k_traverse(ResArgs a) {
     }
 
     uint64_t m_unvisited = a.m, edges_done = 0;
-    uint32_t iterations = 0, pulls = 0, level = 0, far_turn = 0, late_pulls = 0;
+    u64 front_E = 0;
+    uint32_t iterations = 0, pulls = 0, level = 0, far_turn = 0, pull_turn = 0, late_pulls = 0;
     uint32_t thr = PTG_UNREACHED;
     u64 delta = a.delta, bucket_E = 0;
     if (MODE == 1 && a.use_far) thr = a.base + a.delta;
-    bool bottom_up = false, limit = false;
+    bool bottom_up = false, limit = false, scanned = false;
     int cur = 0;
     while (true) {
         const int slot = level % 3, next = (level + 1) % 3, later = (level + 2) % 3;
@@ -620,53 +750,51 @@ __global__ void __launch_bounds__(kBlock, 4) k_traverse(ResArgs a) {
         const Frontier front = frontier_of(a, cur, slot);
         if (MODE == 2 && level == 0) F = a.n, E = a.m;
         if (F == 0) {
-            if (MODE != 1 || !a.use_far) break;
+            if (MODE != 1 || !a.use_far || thr == PTG_UNREACHED) break;
             // next bucket: parked vertices below the threshold were settled by
-            // the bucket that ends; the least of the others sets the new one
+            // the bucket that ends; of the others, those below the next
+            // threshold are its frontier.  A bucket without any is tried once
+            // more from the least parked distance, which this pass finds too.
+            u64 from = thr;
+            if (scanned) {
+                from = ctl->far_min[(far_turn + 2) % 3];
+                if (from == ~0ull) break;
+            } else {
+                // a bucket with few edges costs its passes over the parked
+                // vertices, not its relaxations: wider ones from here on
+                if (bucket_E < max(kWideEdges, (u64)a.n / 2)) delta *= 2;
+                bucket_E = 0;
+            }
+            scanned = true;
+            const uint32_t to = from + delta >= PTG_UNREACHED ? PTG_UNREACHED : (uint32_t)(from + delta);
+            if (leader) ctl->far_min[(far_turn + 1) % 3] = ~0ull;
             uint32_t best = PTG_UNREACHED;
             for (uint64_t w0 = (tid >> 5) * 32; w0 < words; w0 += nthreads) {
                 const uint64_t wd = w0 + lane_id();
                 uint32_t word = wd < words ? a.far_bm[wd] : 0u;
                 const uint32_t had = word;
                 for_words(word, [&](int i, uint32_t bits) {
-                    const bool on = (bits >> lane_id()) & 1u;
-                    const uint32_t d = on ? a.value[(w0 + i) * 32 + lane_id()] : PTG_UNREACHED;
-                    if (d >= thr) best = min(best, d);
-                    const uint32_t keep = __ballot_sync(0xffffffffu, on && d >= thr);
-                    if ((int)lane_id() == i) word = keep;
-                });
-                if (word != had) a.far_bm[wd] = word;
-            }
-            best = __reduce_min_sync(0xffffffffu, best);
-            if (lane_id() == 0 && best != PTG_UNREACHED) atomicMin(&ctl->far_min[far_turn & 1], (u64)best);
-            if (!grid_barrier(ctl)) return;
-            const u64 fm = ctl->far_min[far_turn & 1];
-            if (fm == ~0ull) break;
-            if (leader) ctl->far_min[(far_turn & 1) ^ 1] = ~0ull;
-            far_turn++;
-            // a bucket with few edges costs its passes over the parked
-            // vertices, not its relaxations: wider ones from here on
-            if (bucket_E < max(kWideEdges, (u64)a.n / 2)) delta *= 2;
-            bucket_E = 0;
-            thr = fm + delta >= PTG_UNREACHED ? PTG_UNREACHED : (uint32_t)(fm + delta);
-            for (uint64_t w0 = (tid >> 5) * 32; w0 < words; w0 += nthreads) {
-                const uint64_t wd = w0 + lane_id();
-                uint32_t word = wd < words ? a.far_bm[wd] : 0u;
-                const uint32_t had = word;
-                for_words(word, [&](int i, uint32_t bits) {
                     const uint32_t v = (uint32_t)((w0 + i) * 32 + lane_id());
-                    const bool near = ((bits >> lane_id()) & 1u) && a.value[v] < thr;
+                    const uint32_t d = (bits >> lane_id()) & 1u ? a.value[v] : 0u;
+                    const bool near = d >= thr && d < to;
+                    if (near) buf.least = min(buf.least, d);
+                    else if (d >= thr) best = min(best, d);
                     buf_add(buf, near, v);
-                    const uint32_t moved = __ballot_sync(0xffffffffu, near);
-                    if ((int)lane_id() == i) word = bits & ~moved;
+                    const uint32_t stay = __ballot_sync(0xffffffffu, d >= thr && !near);
+                    if ((int)lane_id() == i) word = stay;
                     while (buf.cnt >= 64) buf_flush<OffT>(buf, a, front);
                 });
                 if (word != had) a.far_bm[wd] = word;
             }
+            best = __reduce_min_sync(0xffffffffu, best);
+            if (lane_id() == 0 && best != PTG_UNREACHED) atomicMin(&ctl->far_min[far_turn % 3], (u64)best);
             buf_finish<OffT>(buf, a, front, &ctl->found[slot], &ctl->edges[slot]);
+            thr = to;
+            far_turn++;
             if (!grid_barrier(ctl)) return;
             continue;
         }
+        scanned = false;
         if (iterations >= a.max_iters) {
             limit = true;
             break;
@@ -676,6 +804,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_traverse(ResArgs a) {
             ctl->few[later] = ctl->items[later] = ctl->bigs[later] = ctl->found[later] = ctl->edges[later] = 0;
             ctl->chunk[(level + 1) & 1] = 0;
             ctl->cands[(level + 1) & 3] = 0;
+            ctl->least[later] = PTG_UNREACHED;
         }
         if (MODE == 0 && a.nz) {
             const u64 seen_E = level ? E : 0;  // the seed level runs top-down
@@ -690,7 +819,56 @@ __global__ void __launch_bounds__(kBlock, 4) k_traverse(ResArgs a) {
             m_unvisited = m_unvisited > seen_E ? m_unvisited - seen_E : 0;
         }
         uint32_t *bm_cur = a.bm[cur], *bm_next = a.bm[cur ^ 1];
-        if (MODE == 0 && bottom_up) {
+        bool sssp_pull = false;
+        u64 pull_E = 0;
+        uint32_t above = 0;
+        int turn = 0;
+        if (MODE == 1) {
+            front_E += E;
+            // A heavy round may look at fewer edges from the other side: only
+            // vertices above the frontier's least distance plus the least
+            // weight can improve.  Their edges are counted first, 35 us on RMAT-24
+            // (not when those of all vertices that were in no frontier are too
+            // many already).  An edge costs both ways about the same, listing
+            // the vertices a quarter of a heavy round: RMAT-24's rounds pull
+            // 119 M edges instead of 307 M in 730 us (1170), 32 M instead of
+            // 56 M in 350 us (430), and push 46 M against 45 M.
+            const u64 most = E / 4 * 3;
+            if (a.can_pull && E > max((u64)kSsspPullEdges, (u64)a.m / 16) && (front_E > a.m || a.m - front_E < most)) {
+                const uint32_t least = ctl->least[slot];
+                above = least + min(a.min_weight, PTG_UNREACHED - 1 - least);
+                turn = pull_turn++ & 1;
+                u64 sum = 0;
+                for (uint64_t v = tid; v < a.n; v += nthreads * 4) {
+                    uint32_t d[4];
+#pragma unroll
+                    for (int i = 0; i < 4; i++) d[i] = v + i * nthreads < a.n ? a.value[v + i * nthreads] : 0u;
+#pragma unroll
+                    for (int i = 0; i < 4; i++)
+                        if (d[i] > above) sum += (u64)(off[v + i * nthreads + 1] - off[v + i * nthreads]);
+                }
+                sum = block_reduce_sum(sum);
+                if (threadIdx.x == 0 && sum) atomicAdd(&ctl->pull_edges[turn], sum);
+                if (!grid_barrier(ctl)) return;
+                pull_E = ctl->pull_edges[turn];
+                sssp_pull = pull_E < most;
+                if (leader) ctl->pull_edges[turn ^ 1] = ctl->pull_items[turn ^ 1] = ctl->pull_bigs[turn ^ 1] = 0;
+            }
+        }
+        if (MODE == 1 && sssp_pull) {
+            pulls++;
+            edges_done += pull_E;
+            bucket_E += E;
+            for (uint64_t i = tid; i < words; i += nthreads) bm_cur[i] = 0u;
+            // its lists go where the frontier's were
+            const Frontier look{a.few[cur], a.q[cur], a.big[cur], &ctl->pull_items[turn] /* (none) */,
+                                &ctl->pull_items[turn], &ctl->pull_bigs[turn], nullptr};
+            const Frontier nx = frontier_of(a, cur ^ 1, next);
+            WarpBuf longer{s_look[wid], 0, PTG_UNREACHED, 0, 0};
+            sssp_pull_few<OffT>(a, above, thr, bm_next, nx, buf, look, longer);
+            if (!grid_barrier(ctl)) return;
+            sssp_pull_longer<OffT>(a, look, thr, bm_next, nx, buf, &ctl->found[next], &ctl->edges[next]);
+        } else if (MODE == 0 && bottom_up) {
             // few unvisited vertices left: what the last pull round looked at and did not find
             const bool late = level && !queued && (ctl->cands[(level + 3) & 3] - F) * 64 < a.n;
             pulls++;
@@ -859,6 +1037,10 @@ void run_resident(ptg_graph *g, TravKind kind, uint32_t src, uint32_t *d_value, 
     if (a.use_far) {
         ws.farbm.ensure(words * 4);
         a.far_bm = ws.farbm.as<uint32_t>();
+    }
+    if (kind == TRAV_SSSP && allow_pull) {
+        a.can_pull = 1;
+        a.min_weight = g->min_weight;
     }
     LevelMsg done{};
     try {

@@ -143,6 +143,7 @@ ptg_graph *make_view(ptg_graph *g, ptg_ctx *lane) {
     v->n_pr_items = g->n_pr_items;
     v->pr_bins_built = g->pr_bins_built;
     v->mean_weight = g->mean_weight;
+    v->min_weight = g->min_weight;
     v->weights_symmetric = g->weights_symmetric;
     v->resident_edges = g->resident_edges;
     v->device_bytes = 0;

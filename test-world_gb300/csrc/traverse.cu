@@ -307,13 +307,18 @@ __global__ void __launch_bounds__(kBlock, 4) k_expand(const uint32_t *q, const O
     }
 }
 
-// Sum of the resident edge weights (for the default near/far bucket width).
+// Sum and least of the resident edge weights (out[0], out[1]).
 __global__ void __launch_bounds__(kBlock) k_weight_sum(const uint32_t *w, uint64_t m, unsigned long long *out) {
     unsigned long long s = 0;
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < m; i += (uint64_t)gridDim.x * blockDim.x)
+    uint32_t least = 0xFFFFFFFFu;
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < m; i += (uint64_t)gridDim.x * blockDim.x) {
         s += w[i];
+        least = min(least, w[i]);
+    }
     s = block_reduce_sum(s);
     if (threadIdx.x == 0 && s) atomicAdd(out, s);
+    least = __reduce_min_sync(0xffffffffu, least);
+    if (lane_id() == 0) atomicMin(out + 1, (unsigned long long)least);
 }
 
 constexpr uint64_t kHotSmemParts = 4096;  // partitions counted in shared memory by k_mark_partitions
@@ -455,43 +460,99 @@ __global__ void __launch_bounds__(kBlock) k_relax_partition(uint64_t e_begin, ui
     }
 }
 
-// Sum over the edges u < v of a hash of (u, v, w), less the same over the
-// edges u > v: zero when the two lists of (smaller end, larger end, weight) are
-// the same (and, where they differ, with probability 2^-64).  Edge-centric
-// tiles; a thread walks the rows of its 8 consecutive edges in registers.
+// Whether every edge carries the same weight both ways: sum over the edges
+// u < v of a hash of (u, v, w), less the same over the edges u > v; zero when the
+// two lists of (smaller end, larger end, weight) are the same (and, where they
+// differ, with probability 2^-64).  Also the weights' sum and minimum, as
+// k_weight_sum.  A warp walks an equal run of edges, 8 consecutive ones per
+// lane and step; the rows that begin in a step's 256 edges are written at their
+// first edge in shared memory, and a running maximum gives each edge its row.
+// (Tiles of a CTA with a search of their row bounds each: 3.07 ms on RMAT-24,
+// 1.83 now; half of it is the hash.)
+constexpr uint32_t kBalStep = 256;
 template <class OffT>
-__global__ void __launch_bounds__(kBlock) k_weight_balance(uint64_t m, uint64_t n, const OffT *off, const uint32_t *col,
-                                                           const uint32_t *w, unsigned long long *out) {
-    __shared__ OffT s_off[kTile + 2];
-    unsigned long long sum = 0;
-    const uint64_t ntiles = (m + kTile - 1) / kTile;
-    for (uint64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        const uint64_t t0 = tile * kTile, t1 = min(m, t0 + kTile);
-        const uint64_t r0 = block_last_le(off, 0, n, t0), r1 = block_last_le(off, r0, n, t1 - 1);
-        const uint64_t nrows = r1 - r0 + 1;
-        const bool staged = nrows <= (uint64_t)kTile;
-        if (staged)
-            for (uint64_t k = threadIdx.x; k <= nrows; k += kBlock) s_off[k] = off[r0 + k];
-        __syncthreads();
-        const uint64_t j0 = t0 + threadIdx.x * (kTile / kBlock);
-        uint64_t row = 0;
-        if (j0 < t1) row = staged ? last_le(s_off, 0, nrows, j0) : last_le(off, r0, r0 + nrows, j0) - r0;
-        for (int i = 0; i < kTile / kBlock; i++) {
-            const uint64_t j = j0 + i;
-            if (j >= t1) break;
-            while (j >= (uint64_t)(staged ? s_off[row + 1] : off[r0 + row + 1])) row++;
-            const unsigned long long u = r0 + row, v = col[j];
-            unsigned long long h = (min(u, v) << 32 | max(u, v)) * 0x9E3779B97F4A7C15ull;
-            h = (h ^ (h >> 29) ^ ((unsigned long long)w[j] << 20)) * 0xBF58476D1CE4E5B9ull;
-            h = (h ^ (h >> 32) ^ w[j]) * 0x94D049BB133111EBull;
-            h ^= h >> 31;
+__global__ void __launch_bounds__(kBlock, 4) k_weight_balance(uint64_t m, uint64_t n, const OffT *off, const uint32_t *col,
+                                                              const uint32_t *w, unsigned long long *out) {
+    constexpr int kEach = kBalStep / 32;
+    __shared__ __align__(16) uint32_t s_row[kBlock / 32][kBalStep];
+    uint32_t *rows = s_row[threadIdx.x >> 5];
+    const unsigned lane = lane_id();
+    const uint64_t warps = (uint64_t)gridDim.x * (kBlock / 32), warp = (uint64_t)blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5);
+    const uint64_t share = ((m + warps - 1) / warps + kBalStep - 1) / kBalStep * kBalStep;
+    const uint64_t end = min(m, (warp + 1) * share);
+    unsigned long long sum = 0, total = 0;
+    uint32_t least = 0xFFFFFFFFu, row = 0;  // row: the last that begins at or before the step's first edge
+    if (warp * share < end) row = (uint32_t)last_le(off, (uint64_t)0, n, warp * share);
+    for (uint64_t t = warp * share; t < end; t += kBalStep) {
+        const uint64_t t1 = min(m, t + kBalStep), j0 = t + lane * kEach;
+        uint32_t vs[kEach], ws[kEach];
+        if (j0 + kEach <= t1) {  // (the arrays start on 256 bytes and j0 is a multiple of 8)
+#pragma unroll
+            for (int i = 0; i < kEach; i += 4) {
+                const uint4 x = *reinterpret_cast<const uint4 *>(col + j0 + i), y = *reinterpret_cast<const uint4 *>(w + j0 + i);
+                vs[i] = x.x, vs[i + 1] = x.y, vs[i + 2] = x.z, vs[i + 3] = x.w;
+                ws[i] = y.x, ws[i + 1] = y.y, ws[i + 2] = y.z, ws[i + 3] = y.w;
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < kEach; i++) {
+                vs[i] = j0 + i < t1 ? col[j0 + i] : 0u;
+                ws[i] = j0 + i < t1 ? w[j0 + i] : 0xFFFFFFFFu;
+            }
+        }
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < kEach; i += 4) *reinterpret_cast<uint4 *>(rows + lane * kEach + i) = make_uint4(0, 0, 0, 0);
+        __syncwarp();
+        // 128 row starts at a time: the runs of short rows would otherwise take
+        // most of the time, a dependent load per 32 rows
+        uint64_t r = (uint64_t)row + 1;
+        for (int c = 128; c == 128; r += c) {
+            uint64_t x[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++) x[i] = r + 32 * i + lane < n ? (uint64_t)off[r + 32 * i + lane] : t1;
+            c = 0;
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const bool in = x[i] < t1;
+                // (of several rows that begin at one edge all but the last are empty)
+                if (in) atomicMax(&rows[x[i] - t], (uint32_t)(r + 32 * i + lane));
+                c += __popc(__ballot_sync(0xffffffffu, in));
+            }
+        }
+        __syncwarp();
+        uint32_t at[kEach], last = 0;
+#pragma unroll
+        for (int i = 0; i < kEach; i++) at[i] = last = max(last, rows[lane * kEach + i]);
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, last, o);
+            if (lane >= (unsigned)o) last = max(last, y);
+        }
+        uint32_t before = __shfl_up_sync(0xffffffffu, last, 1);
+        before = lane ? max(before, row) : row;
+#pragma unroll
+        for (int i = 0; i < kEach; i++) {
+            least = min(least, ws[i]);
+            if (j0 + i >= t1) continue;
+            const uint32_t u = max(at[i], before), v = vs[i];
+            unsigned long long h = ((unsigned long long)min(u, v) << 32 | max(u, v)) * 0x9E3779B97F4A7C15ull;
+            h = (h ^ (h >> 32) ^ ws[i]) * 0xBF58476D1CE4E5B9ull;
+            h = (h ^ (h >> 32)) * 0x94D049BB133111EBull;
+            h ^= h >> 32;
             if (u < v) sum += h;
             if (u > v) sum -= h;
+            total += ws[i];
         }
-        __syncthreads();
+        row = (uint32_t)(r - 1);
     }
     sum = block_reduce_sum(sum);
     if (threadIdx.x == 0 && sum) atomicAdd(out, sum);
+    __syncthreads();
+    total = block_reduce_sum(total);
+    if (threadIdx.x == 0 && total) atomicAdd(out + 1, total);
+    least = __reduce_min_sync(0xffffffffu, least);
+    if (lane == 0) atomicMin(out + 2, (unsigned long long)least);
 }
 
 // Near/far: smallest distance in the far pile (a bitmap).
@@ -575,20 +636,25 @@ int hot_slot(ptg_graph *g, uint64_t p, uint64_t edges) {
 // ---------------------------------------------------------------------------
 // host driver
 // ---------------------------------------------------------------------------
-// Mean resident edge weight, measured once per graph.
+void set_weight_stats(ptg_graph *g, unsigned long long sum, uint32_t least) {
+    g->mean_weight = std::max(1.0, (double)sum / (double)g->resident_edges);
+    g->min_weight = least;
+}
+
+// Mean and least resident edge weight, measured once per graph.
 void measure_mean_weight(ptg_graph *g) {
     if (g->mean_weight != 0 || g->resident_edges == 0 || !g->weighted) return;
     ptg_ctx *ctx = g->ctx;
     cudaStream_t st = ctx->stream;
     ctx->ws.bsum.ensure(1024 * 8);
     unsigned long long *acc = ctx->ws.bsum.as<unsigned long long>();
-    PTG_CUDA_TRY(cudaMemsetAsync(acc, 0, 8, st));
+    unsigned long long h[2] = {0, 0xFFFFFFFFull};
+    PTG_CUDA_TRY(cudaMemcpyAsync(acc, h, 16, cudaMemcpyHostToDevice, st));
     launch(ctx, "k_weight_sum", k_weight_sum, grid_for(g->resident_edges, kBlock, ctx->sm_count * 8), kBlock, 0, st,
            g->d_w.as<uint32_t>(), g->resident_edges, acc);
-    unsigned long long sum = 0;
-    PTG_CUDA_TRY(cudaMemcpyAsync(&sum, acc, 8, cudaMemcpyDeviceToHost, st));
+    PTG_CUDA_TRY(cudaMemcpyAsync(h, acc, 16, cudaMemcpyDeviceToHost, st));
     PTG_CUDA_TRY(cudaStreamSynchronize(st));
-    g->mean_weight = std::max(1.0, (double)sum / (double)g->resident_edges);
+    set_weight_stats(g, h[0], (uint32_t)h[1]);
 }
 
 template <class OffT>
@@ -870,27 +936,25 @@ bool graph_weights_symmetric(ptg_graph *g) {
             ptg_ctx *ctx = g->ctx;
             cudaStream_t st = ctx->stream;
             ctx->ws.bsum.ensure(1024 * 8);
-            unsigned long long *acc = ctx->ws.bsum.as<unsigned long long>(), sum = 0;
-            PTG_CUDA_TRY(cudaMemsetAsync(acc, 0, 8, st));
-            const int grid = grid_for(g->m, kTile, ctx->sm_count * 8);
+            unsigned long long *acc = ctx->ws.bsum.as<unsigned long long>();
+            unsigned long long h[3] = {0, 0, 0xFFFFFFFFull};
+            PTG_CUDA_TRY(cudaMemcpyAsync(acc, h, 24, cudaMemcpyHostToDevice, st));
+            const int grid = grid_for(g->m, kTile, ctx->sm_count * 4);
             if (g->off64)
                 launch(ctx, "k_weight_balance", k_weight_balance<unsigned long long>, grid, kBlock, 0, st, g->m, g->n,
                        g->d_off.as<unsigned long long>(), g->d_col.as<uint32_t>(), g->d_w.as<uint32_t>(), acc);
             else
                 launch(ctx, "k_weight_balance", k_weight_balance<uint32_t>, grid, kBlock, 0, st, g->m, g->n,
                        g->d_off.as<uint32_t>(), g->d_col.as<uint32_t>(), g->d_w.as<uint32_t>(), acc);
-            PTG_CUDA_TRY(cudaMemcpyAsync(&sum, acc, 8, cudaMemcpyDeviceToHost, st));
+            PTG_CUDA_TRY(cudaMemcpyAsync(h, acc, 24, cudaMemcpyDeviceToHost, st));
             PTG_CUDA_TRY(cudaStreamSynchronize(st));
-            g->weights_symmetric = sum == 0;
+            set_weight_stats(g, h[1], (uint32_t)h[2]);
+            g->weights_symmetric = h[0] == 0;
         }
     }
     return g->weights_symmetric == 1;
 }
 
-double graph_mean_weight(ptg_graph *g) {
-    measure_mean_weight(g);
-    return g->mean_weight;
-}
 
 // Default SSSP bucket width of an in-HBM graph: the tuned multiple (0.75) of
 // the mean edge weight, a quarter of that from 2^25 edges on and up to 4 times
@@ -916,6 +980,8 @@ void run_traversal(ptg_graph *g, TravKind kind, uint32_t src, uint32_t *d_value,
         else traverse_impl<uint32_t>(g, kind, src, d_value, flags, delta, max_iters, rr);
         return;
     }
+    bool pull = g->symmetric && !(flags & (PTG_NO_DIRECTION_OPT | PTG_REFERENCE_SCHEDULE));
+    if (kind == TRAV_SSSP) pull = pull && g->m > kSsspPullEdges && graph_weights_symmetric(g);
     if (kind != TRAV_SSSP || (flags & PTG_REFERENCE_SCHEDULE)) delta = 0;
     else if (delta == 0) delta = default_delta(g);
     if (max_iters == 0) max_iters = (uint32_t)std::min<uint64_t>(0xFFFFFFF0ull, 4 * g->n + 16);
@@ -926,8 +992,7 @@ void run_traversal(ptg_graph *g, TravKind kind, uint32_t src, uint32_t *d_value,
         ws.relab[1].ensure(g->n * 4);
         val = ws.relab[0].as<uint32_t>();
     }
-    run_resident(g, kind, src, val, (flags & PTG_LEVEL_ZERO_BASED) ? 0u : 1u, delta,
-                 g->symmetric && !(flags & (PTG_NO_DIRECTION_OPT | PTG_REFERENCE_SCHEDULE)), max_iters, rr);
+    run_resident(g, kind, src, val, (flags & PTG_LEVEL_ZERO_BASED) ? 0u : 1u, delta, pull, max_iters, rr);
     if (val != d_value) cc_labels_out(g, val, ws.relab[1].as<uint32_t>(), d_value);
     PTG_CUDA_TRY(cudaGetLastError());
 }

@@ -1,6 +1,8 @@
 """The one-launch traversal of in-HBM graphs at its edges: degrees around the
 three work lists and a warp's pieces, one CTA and many, long chains (many
 levels, many buckets), every offset width and vertex order, against the oracle."""
+import functools
+
 import numpy as np
 import pytest
 
@@ -88,3 +90,48 @@ def test_iteration_limit(ptg, ctx):
         o.max_iterations = limit
         assert ptg.lib().ptg_bfs(G.h, s, out.ctypes.data_as(ctypes.c_void_p), ctypes.byref(o)) == want
     assert sorted(out) == list(range(1, 65))
+
+
+@functools.lru_cache(None)
+def core_and_leaves(both_ways, seed):
+    """A source joined to a complete core (8.7 M edges), and leaves on the core with degrees around the
+    pull round's three ways to go over a row: the core is one frontier, and what it could still improve
+    has far fewer edges.  Weights are the same both ways, or not on some edges."""
+    rng = np.random.RandomState(seed)
+    core = 2950
+    degrees = np.concatenate([rng.randint(1, 17, 20011), rng.randint(17, 129, 500), rng.randint(129, 600, 60),
+                              [15, 16, 17, 64, 65, 127, 128, 129, 255, 256, 257, 512, 513]])
+    n = 1 + core + len(degrees) + 5  # five without edges
+    a, b = np.meshgrid(np.arange(core), np.arange(core))
+    keep = a < b
+    src, dst = [np.zeros(core, np.int64), 1 + a[keep]], [1 + np.arange(core), 1 + b[keep]]
+    leaf = np.repeat(np.arange(len(degrees)), degrees)
+    src.append(1 + core + leaf)
+    dst.append(1 + (leaf * 37 + np.arange(len(leaf)) * 3) % core)
+    ids = rng.permutation(n)
+    off, col, _ = csr(n, ids[np.concatenate(src)], ids[np.concatenate(dst)], True, 0)
+    inv = np.argsort(ids)
+    row = np.repeat(np.arange(n), np.diff(off).astype(np.int64))
+    lo, hi = np.minimum(inv[row], inv[col]), np.maximum(inv[row], inv[col])
+    h = (lo * 7919 + hi * 104729) % 61
+    w = np.where(lo == 0, 5 + h % 2, np.where(hi <= core, 20 + h, 1 + h)).astype(np.uint32)
+    if not both_ways:
+        w += ((row < col) & (h < 9)).astype(np.uint32)
+    return off, col, w, int(ids[0])
+
+
+@pytest.mark.parametrize("both_ways", [True, False])
+@pytest.mark.parametrize("wide", [False, True])
+@pytest.mark.parametrize("grouped", [False, True])
+def test_sssp_pull_rounds(ptg, ctx, ctx_grouped, oracle, grouped, wide, both_ways):
+    off, col, w, s = core_and_leaves(both_ways, 11)
+    G = (ctx_grouped if grouped else ctx).graph(off, col, w, symmetric=True, wide_offsets=wide)
+    dist = oracle.sssp(off, col, w, s)
+    for delta in (0, 3, 33, 1000000):
+        st = {}
+        assert (G.sssp(s, delta=delta, stats=st) == dist).all(), delta
+        if delta == 1000000:  # (the core is one frontier)
+            assert (st["bottom_up_rounds"] > 0) == both_ways
+        assert (G.sssp(s, delta=delta, flags=ptg.PTG_NO_DIRECTION_OPT, stats=st) == dist).all(), delta
+        assert st["bottom_up_rounds"] == 0
+    G.close()
