@@ -160,12 +160,12 @@ typedef struct ptg_run_stats {
     uint64_t edges_relaxed;     /* edges inspected by relax kernels                */
     uint64_t vertices_reached;  /* vertices with a finite value                    */
     uint64_t edges_in_component;/* directed edges out of reached vertices          */
-    uint64_t link_bytes;        /* bytes streamed host->device by the swapper      */
-    uint64_t partitions_streamed;
+    uint64_t link_bytes;        /* edge bytes copied or read from host memory      */
+    uint64_t partitions_streamed;/* active partitions copied or read in place      */
     uint64_t partitions_skipped;/* streamed partitions skipped as inactive         */
     uint64_t partitions_cached; /* active partitions served from the hot cache     */
     double device_ms;           /* GPU time of the run (CUDA events)              */
-    double link_ms;             /* time the copy stream was busy                   */
+    double link_ms;             /* time the link was busy with them               */
 } ptg_run_stats;
 
 typedef struct ptg_run_opts {

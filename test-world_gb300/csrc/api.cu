@@ -36,6 +36,27 @@ void stream_edges(ptg_graph *g, int which, void *dst, uint64_t e0, uint64_t e1, 
     }
 }
 
+// Device address of h_col (which = 0) or h_w (1), or nullptr unless every
+// streamed partition in the page-locked range is mapped where the first one says.
+const uint32_t *mapped_edges(ptg_graph *g, int which) {
+    const uint32_t *base = which ? g->h_w : g->h_col;
+    const uintptr_t lo = std::max(g->pin_lo[which], (uintptr_t)(base + g->resident_edges));
+    const uintptr_t hi = std::min(g->pin_hi[which], (uintptr_t)(base + g->m));
+    uintptr_t shift = 0;
+    for (uintptr_t a = lo; a < hi; a += g->partition_edges * 4) {
+        for (uintptr_t x : {a, std::min(a + g->partition_edges * 4, hi) - 4}) {
+            void *d = nullptr;
+            if (cudaHostGetDevicePointer(&d, (void *)x, 0) != cudaSuccess) {
+                cudaGetLastError();
+                return nullptr;
+            }
+            if (x == lo) shift = (uintptr_t)d - x;
+            if ((uintptr_t)d - x != shift) return nullptr;
+        }
+    }
+    return lo < hi ? (const uint32_t *)((uintptr_t)base + shift) : nullptr;
+}
+
 void set_error(ptg_ctx *ctx, const Error &e) {
     if (ctx) ctx->last_error = e.msg;
 }
@@ -484,6 +505,8 @@ void ptg_graph_destroy(ptg_graph *g) {
     }
     for (int i = 0; i < 2; i++)
         if (g->link_ev[i]) cudaEventDestroy(g->link_ev[i]);
+    if (g->direct_done) cudaEventDestroy(g->direct_done);
+    if (g->hits_ready) cudaEventDestroy(g->hits_ready);
     delete g;
 }
 
@@ -724,6 +747,10 @@ ptg_status ptg_graph_create(ptg_ctx *ctx, const ptg_csr *csr, const ptg_partitio
                 PTG_CUDA_TRY(cudaEventCreateWithFlags(&g->stage_free[b], cudaEventDisableTiming));
                 if (b < 2) PTG_CUDA_TRY(cudaEventCreate(&g->link_ev[b]));
             }
+            PTG_CUDA_TRY(cudaEventCreateWithFlags(&g->direct_done, cudaEventDisableTiming));
+            PTG_CUDA_TRY(cudaEventCreateWithFlags(&g->hits_ready, cudaEventDisableTiming));
+            g->dev_col = mapped_edges(g, 0);
+            if (g->weighted) g->dev_w = mapped_edges(g, 1);
             g->device_bytes += (uint64_t)g->n_stage * PE * bpe;
             g->part_visits.assign(P, 0);
             if (g->cache_slots) {
@@ -733,8 +760,6 @@ ptg_status ptg_graph_create(ptg_ctx *ctx, const ptg_csr *csr, const ptg_partitio
                     PTG_CUDA_TRY(cudaEventCreateWithFlags(&g->slots[i].freed, cudaEventDisableTiming));
                 }
                 g->slot_of.assign(P, -1);
-                g->d_part_hits.ensure(P * 8);
-                g->h_part_hits.ensure(P * 8);
                 g->device_bytes += (uint64_t)g->cache_slots * PE * bpe;  // taken as partitions turn hot
                 if (g->cache_static) place_hubs(g, host_offsets(csr), PE, st);
             }

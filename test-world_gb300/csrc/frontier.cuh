@@ -19,7 +19,7 @@ namespace {
 // offset loads in flight together.
 constexpr int kScanItems = 4;
 template <class OffT>
-__device__ __forceinline__ unsigned long long scan_items(const uint32_t *q, const OffT *off, OffT clip, uint64_t i0,
+__device__ __forceinline__ unsigned long long scan_items(const uint32_t *q, const OffT *off, OffT from, OffT clip, uint64_t i0,
                                                          uint64_t hi, OffT (&d)[kScanItems], OffT (&st)[kScanItems]) {
     uint32_t u[kScanItems];
 #pragma unroll
@@ -27,7 +27,7 @@ __device__ __forceinline__ unsigned long long scan_items(const uint32_t *q, cons
     OffT e[kScanItems];
 #pragma unroll
     for (int k = 0; k < kScanItems; k++) {
-        st[k] = i0 + k < hi ? off[u[k]] : (OffT)0;
+        st[k] = i0 + k < hi ? max(off[u[k]], from) : (OffT)0;
         e[k] = i0 + k < hi ? off[u[k] + 1] : (OffT)0;
     }
     unsigned long long t = 0;
@@ -43,7 +43,7 @@ __device__ __forceinline__ unsigned long long scan_items(const uint32_t *q, cons
 // Pass 1 of the frontier degree scan: per-CTA sums over contiguous slices.
 template <class OffT>
 __global__ void __launch_bounds__(kBlock) k_scan_reduce(const uint32_t *q, const TravCtl *ctl,
-                                                        const OffT *off, OffT clip,
+                                                        const OffT *off, OffT from, OffT clip,
                                                         unsigned long long *bsum) {
     uint64_t F = ctl->F;
     uint64_t per = (F + gridDim.x - 1) / gridDim.x;
@@ -51,7 +51,7 @@ __global__ void __launch_bounds__(kBlock) k_scan_reduce(const uint32_t *q, const
     unsigned long long s = 0;
     for (uint64_t i = lo + threadIdx.x * kScanItems; i < hi; i += kBlock * kScanItems) {
         OffT d[kScanItems], st[kScanItems];
-        s += scan_items(q, off, clip, i, hi, d, st);
+        s += scan_items(q, off, from, clip, i, hi, d, st);
     }
     s = block_reduce_sum(s);
     if (threadIdx.x == 0) bsum[blockIdx.x] = s;
@@ -59,7 +59,7 @@ __global__ void __launch_bounds__(kBlock) k_scan_reduce(const uint32_t *q, const
 
 // Pass 2: one CTA turns the per-CTA sums into exclusive offsets; ctl->E = total.
 __global__ void __launch_bounds__(kBlock) k_scan_bsums(unsigned long long *bsum, int nb,
-                                                       TravCtl *ctl) {
+                                                       TravCtl *ctl, int count) {
     unsigned long long carry = 0;
     for (int base = 0; base < nb; base += kBlock) {
         int i = base + threadIdx.x;
@@ -70,7 +70,7 @@ __global__ void __launch_bounds__(kBlock) k_scan_bsums(unsigned long long *bsum,
     }
     if (threadIdx.x == 0) {
         ctl->E = carry;
-        ctl->edges_done += carry;
+        if (count) ctl->edges_done += carry;
     }
 }
 
@@ -78,7 +78,7 @@ __global__ void __launch_bounds__(kBlock) k_scan_bsums(unsigned long long *bsum,
 // clipped degrees), rs[i] (adjacency start of q[i]) and sc[F] = E.
 template <class OffT>
 __global__ void __launch_bounds__(kBlock) k_scan_write(const uint32_t *q, const TravCtl *ctl,
-                                                       const OffT *off, OffT clip,
+                                                       const OffT *off, OffT from, OffT clip,
                                                        const unsigned long long *bsum, OffT *sc,
                                                        OffT *rs) {
     uint64_t F = ctl->F;
@@ -89,7 +89,7 @@ __global__ void __launch_bounds__(kBlock) k_scan_write(const uint32_t *q, const 
         const uint64_t i0 = base + threadIdx.x * kScanItems;
         OffT d[kScanItems], st[kScanItems];
         unsigned long long tot;
-        unsigned long long ex = block_exclusive_scan(scan_items(q, off, clip, i0, hi, d, st), tot);
+        unsigned long long ex = block_exclusive_scan(scan_items(q, off, from, clip, i0, hi, d, st), tot);
 #pragma unroll
         for (int k = 0; k < kScanItems; k++) {
             if (i0 + k < hi) {
@@ -111,7 +111,8 @@ constexpr uint32_t kSmallFrontier = 16384;
 // entry), and tr[ntiles] = F - 1, as last_le gives them.
 template <class OffT>
 __global__ void __launch_bounds__(kBlock) k_scan_small(const uint32_t *q, TravCtl *ctl, const OffT *off,
-                                                       OffT clip, OffT *sc, OffT *rs, uint32_t *tr) {
+                                                       OffT from, OffT clip, OffT *sc, OffT *rs, uint32_t *tr,
+                                                       int count) {
     uint64_t F = ctl->F;
     unsigned long long run = 0;
     const unsigned lane = lane_id();
@@ -119,7 +120,7 @@ __global__ void __launch_bounds__(kBlock) k_scan_small(const uint32_t *q, TravCt
         const uint64_t i0 = base + threadIdx.x * kScanItems;
         OffT d[kScanItems], st[kScanItems];
         unsigned long long tot;
-        unsigned long long ex = block_exclusive_scan(scan_items(q, off, clip, i0, F, d, st), tot);
+        unsigned long long ex = block_exclusive_scan(scan_items(q, off, from, clip, i0, F, d, st), tot);
         unsigned long long t_lo[kScanItems], t_hi[kScanItems];
 #pragma unroll
         for (int k = 0; k < kScanItems; k++) {
@@ -151,7 +152,7 @@ __global__ void __launch_bounds__(kBlock) k_scan_small(const uint32_t *q, TravCt
     if (threadIdx.x == 0) {
         sc[F] = (OffT)run;
         ctl->E = run;
-        ctl->edges_done += run;
+        if (count) ctl->edges_done += run;
         if (tr) tr[(run + kTile - 1) / kTile] = (uint32_t)(F ? F - 1 : 0);
     }
 }

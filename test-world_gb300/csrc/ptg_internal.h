@@ -317,6 +317,8 @@ struct ptg_graph {
     const uint32_t *h_col = nullptr, *h_w = nullptr;  // pinned host edge arrays
     // page-locked address range of h_col / h_w (bytes outside it are pageable)
     uintptr_t pin_lo[2] = {0, 0}, pin_hi[2] = {~(uintptr_t)0, ~(uintptr_t)0};
+    // where kernels read h_col / h_w in place (by edge index; nullptr: they cannot)
+    const uint32_t *dev_col = nullptr, *dev_w = nullptr;
     std::vector<void *> registered;                    // cudaHostRegister'ed ranges
     ptg::PinnedBuf own_col, own_w;                     // owned pinned copies
     ptg::DevBuf stage_col[3], stage_w[3];
@@ -324,6 +326,8 @@ struct ptg_graph {
     cudaEvent_t stage_ready[3] = {nullptr, nullptr, nullptr};
     cudaEvent_t stage_free[3] = {nullptr, nullptr, nullptr};
     cudaEvent_t link_ev[2] = {nullptr, nullptr};  // first copy start / last copy end of a level
+    cudaEvent_t hits_ready = nullptr;             // a level's active edges per partition are on the host
+    cudaEvent_t direct_done = nullptr;            // a level's reads of host memory in place
     uint64_t device_bytes = 0;
     // hot-partition residency
     uint32_t resident_policy = PTG_RESIDENT_PREFIX;
@@ -333,8 +337,6 @@ struct ptg_graph {
     bool cache_static = false;            // slots filled at creation, no promotion (_HUBS)
     std::unique_ptr<ptg::HotSlot[]> slots;
     std::vector<int> slot_of;             // [P] slot of a cached partition, -1 if none
-    ptg::DevBuf d_part_hits;              // u64[P] per level (k_mark_partitions)
-    ptg::PinnedBuf h_part_hits;
 };
 
 namespace ptg {

@@ -31,12 +31,15 @@
 //  * SSSP with a bucket width keeps a near frontier below a moving threshold
 //    and a far pile above it.
 //  * Edges past the resident prefix live in pinned host memory
-//    and are cut into fixed-size partitions.  Each round only partitions that
-//    hold an active vertex's edges are copied (cudaMemcpyAsync on a copy
-//    stream into 2-3 staging buffers, ordered with events) and relaxed
-//    edge-centrically; the rest are skipped (reference: 20 CPU threads gather
-//    active adjacency into a unified-memory buffer the GPU page-faults on,
-//    main.cu:1126-1156, 1336-1378).
+//    and are cut into fixed-size partitions.  Each round the active edges of
+//    every partition are counted.  Mostly active partitions are copied
+//    (cudaMemcpyAsync on a copy stream into 2-3 staging buffers, ordered with
+//    events) and relaxed edge-centrically, those with few active edges are read
+//    in place by a kernel, row by row, and the rest are skipped (reference: 20
+//    CPU threads gather active adjacency into a unified-memory buffer the GPU
+//    page-faults on, main.cu:1126-1156, 1336-1378).  The count is on the host
+//    while the resident edges are relaxed, so copies start meanwhile.  SSSP of
+//    a directed RMAT-22 with half of its edges streamed: 12.2 -> 5.9 ms.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -328,14 +331,13 @@ constexpr uint64_t kHotSmemParts = 4096;  // partitions counted in shared memory
 // flags 4096-edge fragments of active vertices).
 template <class OffT>
 __global__ void k_mark_partitions(const uint32_t *q, const TravCtl *ctl, const OffT *off,
-                                  uint64_t resident_edges, uint64_t part_edges,
-                                  uint64_t resident_parts, uint64_t nparts, uint8_t *flags,
+                                  uint64_t resident_edges, uint64_t part_edges, uint64_t nparts,
                                   unsigned long long *hits) {
-    // hits (hot-partition cache only): edges of frontier vertices per
-    // partition this level, summed per CTA in shared memory when the
-    // partition count allows (the dynamic shared size is then nparts * 8)
+    // hits: edges of frontier vertices per partition this level, summed per
+    // CTA in shared memory when the partition count allows (the dynamic shared
+    // size is then nparts * 8)
     extern __shared__ unsigned long long s_hits[];
-    const bool local = hits != nullptr && nparts <= kHotSmemParts;
+    const bool local = nparts <= kHotSmemParts;
     if (local) {
         for (uint64_t i = threadIdx.x; i < nparts; i += blockDim.x) s_hits[i] = 0;
         __syncthreads();
@@ -349,12 +351,9 @@ __global__ void k_mark_partitions(const uint32_t *q, const TravCtl *ctl, const O
         if (b < resident_edges) b = resident_edges;
         uint64_t p0 = b / part_edges, p1 = (e - 1) / part_edges;
         for (uint64_t p = p0; p <= p1 && p < nparts; p++) {
-            if (p >= resident_parts && !flags[p]) flags[p] = 1;
-            if (hits) {
-                uint64_t lo = max(b, p * part_edges), hi = min(e, (p + 1) * part_edges);
-                if (local) atomicAdd(&s_hits[p], (unsigned long long)(hi - lo));
-                else atomicAdd(&hits[p], (unsigned long long)(hi - lo));
-            }
+            uint64_t lo = max(b, p * part_edges), hi = min(e, (p + 1) * part_edges);
+            if (local) atomicAdd(&s_hits[p], (unsigned long long)(hi - lo));
+            else atomicAdd(&hits[p], (unsigned long long)(hi - lo));
         }
     }
     if (local) {
@@ -374,6 +373,49 @@ __global__ void k_mark_partitions(const uint32_t *q, const TravCtl *ctl, const O
 template <int MODE>
 __device__ __forceinline__ bool part_active(const uint32_t *bm_cur, const PushTargets &t, uint32_t u) {
     return bit_test(bm_cur, u) || (MODE != 0 && bit_test(t.bm_next, u));
+}
+
+// Out-of-core: relaxes the frontier's streamed edges where they lie in host
+// memory, in the partitions that `direct` names, so that only their rows cross
+// the link.  Tiles of the scanned rows as k_expand, but a warp reads neighbouring
+// edges with each load, so a row arrives in whole sectors.  Bound by the link:
+// 160-200 GB/s on RMAT rows of 16 edges, where copies reach 211.
+template <class OffT, int MODE>
+__global__ void __launch_bounds__(kBlock) k_expand_host(const uint32_t *q, const OffT *sc, const OffT *rs,
+                                                        const uint32_t *tr, const uint32_t *col, const uint32_t *w,
+                                                        const uint8_t *direct, uint64_t part_edges, PushTargets t) {
+    const uint64_t E = t.ctl->E, ntiles = (E + kTile - 1) / kTile;
+    const uint32_t thr = t.ctl->threshold;
+    for (uint64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+        const uint64_t t1 = min(E, (tile + 1) * kTile), r0 = tr[tile], r1 = (uint64_t)tr[tile + 1] + 1;
+        uint64_t e[kItems];
+        uint32_t uval[kItems], v[kItems], nd[kItems];
+#pragma unroll
+        for (int b = 0; b < kItems; b++) {
+            const uint64_t j = tile * kTile + b * kBlock + threadIdx.x;
+            e[b] = ~0ull;
+            uval[b] = 0;
+            if (j < t1) {
+                const uint64_t row = last_le(sc, r0, r1, j);
+                const uint64_t x = (uint64_t)rs[row] + (j - (uint64_t)sc[row]);
+                if (direct[x / part_edges]) {
+                    e[b] = x;
+                    uval[b] = t.value[q[row]];
+                }
+            }
+        }
+#pragma unroll
+        for (int b = 0; b < kItems; b++) {
+            v[b] = e[b] != ~0ull ? __ldcs(col + e[b]) : PTG_UNREACHED;
+            nd[b] = MODE == 1 && e[b] != ~0ull ? __ldcs(w + e[b]) : 0u;
+        }
+#pragma unroll
+        for (int b = 0; b < kItems; b++) {
+            if (v[b] == PTG_UNREACHED) continue;
+            nd[b] = MODE == 0 ? uval[b] + 1u : uval[b] + nd[b];
+            relax_probe(t, v[b], nd[b], thr);
+        }
+    }
 }
 
 // Out-of-core: relax every edge of one staged partition whose source vertex
@@ -605,25 +647,24 @@ __global__ void __launch_bounds__(kBlock) k_far_split(uint32_t *far_bm, uint64_t
 // has fewer visits; a cached partition is relaxed from its slot without a
 // copy, in this and every later traversal of the graph.  Returns the slot,
 // or -1 to use a staging buffer.
-int hot_slot(ptg_graph *g, uint64_t p, uint64_t edges) {
-    if (g->slot_of[p] >= 0) return g->slot_of[p];
+int hot_victim(const ptg_graph *g, uint64_t p, uint64_t edges) {
     if (g->cache_static) return -1;
     if ((double)g->part_visits[p] * 4096.0 <= (double)g->hot_threshold * (double)edges) return -1;
     int victim = -1;
     for (uint32_t s = 0; s < g->cache_slots; s++) {
         int64_t q = g->slots[s].part;
-        if (q < 0) {
-            victim = (int)s;
-            break;
-        }
+        if (q < 0) return (int)s;
         if (victim < 0 || g->part_visits[q] < g->part_visits[g->slots[victim].part]) victim = (int)s;
     }
+    return victim >= 0 && g->part_visits[g->slots[victim].part] < g->part_visits[p] ? victim : -1;
+}
+
+int hot_slot(ptg_graph *g, uint64_t p, uint64_t edges) {
+    if (g->slot_of[p] >= 0) return g->slot_of[p];
+    const int victim = hot_victim(g, p, edges);
     if (victim < 0) return -1;
     HotSlot &hs = g->slots[victim];
-    if (hs.part >= 0) {
-        if (g->part_visits[hs.part] >= g->part_visits[p]) return -1;
-        g->slot_of[hs.part] = -1;
-    }
+    if (hs.part >= 0) g->slot_of[hs.part] = -1;
     uint64_t bytes = g->partition_edges * 4;
     hs.col.ensure(bytes);
     if (g->weighted) hs.w.ensure(bytes);
@@ -636,6 +677,36 @@ int hot_slot(ptg_graph *g, uint64_t p, uint64_t edges) {
 // ---------------------------------------------------------------------------
 // host driver
 // ---------------------------------------------------------------------------
+// Whether a kernel may read the edges [e0, e1) in host memory.
+bool readable_in_place(const ptg_graph *g, uint64_t e0, uint64_t e1, bool weights) {
+    auto in = [&](int which, const uint32_t *h, const uint32_t *d) {
+        return d && (uintptr_t)(h + e0) >= g->pin_lo[which] && (uintptr_t)(h + e1) <= g->pin_hi[which];
+    };
+    return in(0, g->h_col, g->dev_col) && (!weights || in(1, g->h_w, g->dev_w));
+}
+
+// Scan of the frontier's degrees, of the edges in [from, to) only: prefix sums
+// and row starts in ws.scan / ws.rowstart, and the row that every tile begins in.
+template <class OffT>
+void scan_frontier(ptg_ctx *ctx, const uint32_t *q, uint64_t F, TravCtl *ctl, const OffT *off, OffT from, OffT to,
+                   bool count, uint32_t *tr) {
+    constexpr int kScanBlocks = 1024;
+    Workspace &ws = ctx->ws;
+    cudaStream_t st = ctx->stream;
+    OffT *sc = ws.scan.as<OffT>(), *rs = ws.rowstart.as<OffT>();
+    if (F <= kSmallFrontier) {  // one CTA: the scan and the tile rows
+        launch(ctx, "k_scan_small", k_scan_small<OffT>, 1, kBlock, 0, st, q, ctl, off, from, to, sc, rs, tr, (int)count);
+        return;
+    }
+    const int blocks = grid_for(F, kBlock, kScanBlocks);
+    ws.bsum.ensure(kScanBlocks * 8);
+    unsigned long long *bsum = ws.bsum.as<unsigned long long>();
+    launch(ctx, "k_scan_reduce", k_scan_reduce<OffT>, blocks, kBlock, 0, st, q, ctl, off, from, to, bsum);
+    launch(ctx, "k_scan_bsums", k_scan_bsums, 1, kBlock, 0, st, bsum, blocks, ctl, (int)count);
+    launch(ctx, "k_scan_write", k_scan_write<OffT>, blocks, kBlock, 0, st, q, ctl, off, from, to, bsum, sc, rs);
+    launch(ctx, "k_tile_rows", k_tile_rows<OffT>, ctx->sm_count * 4, kBlock, 0, st, sc, ctl, tr);
+}
+
 void set_weight_stats(ptg_graph *g, unsigned long long sum, uint32_t least) {
     g->mean_weight = std::max(1.0, (double)sum / (double)g->resident_edges);
     g->min_weight = least;
@@ -674,15 +745,13 @@ void traverse_impl(ptg_graph *g, TravKind kind, uint32_t src, uint32_t *d_value,
     ws.scan.ensure((n + 1) * sizeof(OffT));
     ws.rowstart.ensure((n + 1) * sizeof(OffT));
     ws.tiles.ensure((g->resident_edges / kTile + 4) * sizeof(uint32_t));
-    const int kScanBlocks = 1024;
-    ws.bsum.ensure(kScanBlocks * 8);
     ws.ctl.ensure(sizeof(TravCtl));
     ws.h_ctl.ensure(sizeof(TravCtl));
     // Near/far buckets save edge work in HBM; a streamed graph is bound by the
-    // host link, where every round re-copies its active partitions, so it
+    // host link, and what its rounds read again hardly falls with them, so it
     // relaxes in label-correcting rounds unless a bucket width is asked for
-    // (RMAT-26 all streamed: 9 rounds and 55 GB over the link instead of 18
-    // rounds and 107 GB).
+    // (RMAT-24 all streamed: 9 rounds, 3.9 GB over the link and 21.9 ms, with
+    // buckets of 32 (mean weight) 18 rounds, 3.7 GB and 22.0 ms).
     const bool use_far = kind == TRAV_SSSP && !(flags & PTG_REFERENCE_SCHEDULE) && delta != 0;
     if (use_far) ws.farbm.ensure(words * 4);
     TravCtl *d_ctl = ws.ctl.as<TravCtl>();
@@ -727,9 +796,15 @@ void traverse_impl(ptg_graph *g, TravKind kind, uint32_t src, uint32_t *d_value,
     if (max_iters == 0) max_iters = (uint32_t)std::min<uint64_t>(0xFFFFFFF0ull, 4 * n + 16);
 
     bool link_open = false;  // a level's copies were recorded between link_ev[0] and link_ev[1]
-    ws.flags.ensure(g->num_partitions);
-    ws.h_flags.ensure(g->num_partitions);
-    uint8_t *h_flags = ws.h_flags.as<uint8_t>();
+    // per level and partition: active edges, and whether they are read in place
+    const uint64_t P = g->num_partitions;
+    ws.flags.ensure(P * 9);
+    ws.h_flags.ensure(P * 9);
+    unsigned long long *h_hits = ws.h_flags.as<unsigned long long>();
+    uint8_t *h_direct = reinterpret_cast<uint8_t *>(h_hits + P);
+    unsigned long long *d_hits = ws.flags.as<unsigned long long>();
+    uint8_t *d_direct = reinterpret_cast<uint8_t *>(d_hits + P);
+    const bool need_w = kind == TRAV_SSSP;
     int stage_next = 0;
 
     while (true) {
@@ -772,21 +847,16 @@ void traverse_impl(ptg_graph *g, TravKind kind, uint32_t src, uint32_t *d_value,
         // bm_nxt is clear: zeroed at the start, then by each level's
         // compaction as the bitmap it had just finished with
         PushTargets pt{d_value, bm_nxt, use_far ? ws.farbm.as<uint32_t>() : nullptr, d_ctl};
-        int scan_blocks = grid_for(F, kBlock, kScanBlocks);
-        unsigned long long *bsum = ws.bsum.as<unsigned long long>();
-        OffT *sc = ws.scan.as<OffT>(), *rs = ws.rowstart.as<OffT>();
-        const bool small = F <= kSmallFrontier;
         uint32_t *tr = ws.tiles.as<uint32_t>();
-        if (small) {  // one CTA: the scan and the tile rows
-            launch(ctx, "k_scan_small", k_scan_small<OffT>, 1, kBlock, 0, st, q_cur, d_ctl, off, clip, sc, rs, tr);
-        } else {
-            launch(ctx, "k_scan_reduce", k_scan_reduce<OffT>, scan_blocks, kBlock, 0, st, q_cur, d_ctl, off, clip,
-                   bsum);
-            launch(ctx, "k_scan_bsums", k_scan_bsums, 1, kBlock, 0, st, bsum, scan_blocks, d_ctl);
-            launch(ctx, "k_scan_write", k_scan_write<OffT>, scan_blocks, kBlock, 0, st, q_cur, d_ctl, off, clip, bsum,
-                   sc, rs);
-            launch(ctx, "k_tile_rows", k_tile_rows<OffT>, sms * 4, kBlock, 0, st, sc, d_ctl, tr);
-        }
+        // which partitions hold active edges: known on the host while the
+        // resident edges are relaxed, so that copies start meanwhile
+        PTG_CUDA_TRY(cudaMemsetAsync(d_hits, 0, P * 8, st));
+        launch(ctx, "k_mark_partitions", k_mark_partitions<OffT>, grid_for(F, kBlock, sms * 8), kBlock,
+               P <= kHotSmemParts ? P * 8 : 0, st, q_cur, d_ctl, off, g->resident_edges, g->partition_edges, P, d_hits);
+        PTG_CUDA_TRY(cudaMemcpyAsync(h_hits, d_hits, P * 8, cudaMemcpyDeviceToHost, st));
+        PTG_CUDA_TRY(cudaEventRecord(g->hits_ready, st));
+        scan_frontier<OffT>(ctx, q_cur, F, d_ctl, off, (OffT)0, clip, true, tr);
+        OffT *sc = ws.scan.as<OffT>(), *rs = ws.rowstart.as<OffT>();
         const int eg = sms * (int)ctx->tuning.expand_ctas_per_sm;
         if (kind == TRAV_BFS)
             launch(ctx, "k_expand_bfs", k_expand<OffT, 0>, eg, kBlock, 0, st, q_cur, sc, rs, tr, col, wt, pt);
@@ -798,35 +868,56 @@ void traverse_impl(ptg_graph *g, TravKind kind, uint32_t src, uint32_t *d_value,
         {
             // stream the active partitions past the resident prefix
             const bool hot = g->cache_slots > 0;
-            uint8_t *d_flags = ws.flags.as<uint8_t>();
-            unsigned long long *d_hits = hot ? g->d_part_hits.as<unsigned long long>() : nullptr;
-            PTG_CUDA_TRY(cudaMemsetAsync(d_flags, 0, g->num_partitions, st));
-            if (hot) PTG_CUDA_TRY(cudaMemsetAsync(d_hits, 0, g->num_partitions * 8, st));
-            size_t hsm = hot && g->num_partitions <= kHotSmemParts ? g->num_partitions * 8 : 0;
-            launch(ctx, "k_mark_partitions", k_mark_partitions<OffT>, grid_for(F, kBlock, sms * 8), kBlock,
-                   hsm, st, q_cur, d_ctl, off, g->resident_edges, g->partition_edges,
-                   g->resident_partitions, g->num_partitions, d_flags, d_hits);
-            PTG_CUDA_TRY(cudaMemcpyAsync(h_flags, d_flags, g->num_partitions, cudaMemcpyDeviceToHost, st));
-            if (hot)
-                PTG_CUDA_TRY(cudaMemcpyAsync(g->h_part_hits.p, d_hits, g->num_partitions * 8,
-                                             cudaMemcpyDeviceToHost, st));
-            PTG_CUDA_TRY(cudaStreamSynchronize(st));
+            PTG_CUDA_TRY(cudaEventSynchronize(g->hits_ready));
             link_open = false;
-            const bool need_w = kind == TRAV_SSSP;
-            cudaStream_t cs = ctx->copy_stream;
-            for (uint64_t p = g->resident_partitions; p < g->num_partitions; p++) {
-                if (!h_flags[p]) {
-                    rr.parts_skipped++;
-                    continue;
+            // A partition of which at most three quarters are active is read in
+            // place, else copied.  SSSP of directed RMAT graphs with the line at
+            // (never, 1/4, 1/2, 3/4, 7/8, always): RMAT-22 half streamed 10.9,
+            // 6.2, 4.9, 4.8, 4.8, 5.2 ms; RMAT-24 all streamed 55, 26.6, 21.9,
+            // 21.4, 21.4, 23.3 ms; BFS of the former 4.5, 2.0, 1.9, 1.9, 1.9, 1.9.
+            uint64_t active = 0, direct = 0;  // streamed edges of the frontier; those read in place
+            for (uint64_t p = g->resident_partitions; p < P && hot; p++) g->part_visits[p] += h_hits[p];
+            for (uint64_t p = g->resident_partitions; p < P; p++) {
+                const uint64_t e0 = p * g->partition_edges, e1 = std::min<uint64_t>(g->m, e0 + g->partition_edges);
+                // (what is in a cache slot, or is copied into one now, needs no link)
+                h_direct[p] = h_hits[p] && !(hot && g->slot_of[p] >= 0) && h_hits[p] * 4 <= (e1 - e0) * 3 &&
+                              readable_in_place(g, e0, e1, need_w);
+                rr.parts_skipped += !h_hits[p];
+                active += h_hits[p];
+                if (h_direct[p]) {
+                    direct += h_hits[p];
+                    rr.parts_streamed++;
                 }
+            }
+            if (direct) {
+                ws.tiles.ensure((active / kTile + 4) * sizeof(uint32_t));
+                tr = ws.tiles.as<uint32_t>();
+                std::memset(h_direct, 0, g->resident_partitions);
+                PTG_CUDA_TRY(cudaMemcpyAsync(d_direct, h_direct, P, cudaMemcpyHostToDevice, st));
+                scan_frontier<OffT>(ctx, q_cur, F, d_ctl, off, clip, (OffT)g->m, false, tr);
+                PTG_CUDA_TRY(cudaEventRecord(g->link_ev[0], st));
+                link_open = true;
+                const int hg = grid_for(active, kTile, sms * 8);
+                if (kind == TRAV_BFS)
+                    launch(ctx, "k_expand_host_bfs", k_expand_host<OffT, 0>, hg, kBlock, 0, st, q_cur, sc, rs, tr,
+                           g->dev_col, g->dev_w, d_direct, g->partition_edges, pt);
+                else if (kind == TRAV_SSSP)
+                    launch(ctx, "k_expand_host_sssp", k_expand_host<OffT, 1>, hg, kBlock, 0, st, q_cur, sc, rs, tr,
+                           g->dev_col, g->dev_w, d_direct, g->partition_edges, pt);
+                else
+                    launch(ctx, "k_expand_host_cc", k_expand_host<OffT, 2>, hg, kBlock, 0, st, q_cur, sc, rs, tr,
+                           g->dev_col, g->dev_w, d_direct, g->partition_edges, pt);
+                PTG_CUDA_TRY(cudaGetLastError());
+                PTG_CUDA_TRY(cudaEventRecord(g->direct_done, st));
+                rr.link_bytes += direct * (need_w ? 8 : 4);
+            }
+            cudaStream_t cs = ctx->copy_stream;
+            for (uint64_t p = g->resident_partitions; p < P; p++) {
+                if (!h_hits[p] || h_direct[p]) continue;
                 uint64_t e0 = p * g->partition_edges;
                 uint64_t e1 = std::min<uint64_t>(g->m, e0 + g->partition_edges);
                 const uint32_t *sc_ = nullptr, *sw_ = nullptr;
-                int slot = -1;
-                if (hot) {
-                    g->part_visits[p] += g->h_part_hits.as<unsigned long long>()[p];
-                    slot = hot_slot(g, p, e1 - e0);
-                }
+                const int slot = hot ? hot_slot(g, p, e1 - e0) : -1;
                 // a partition copies into a cache slot (kept for later levels and
                 // queries) or into the next staging buffer
                 bool copy_col = true, copy_w = need_w;
@@ -887,6 +978,7 @@ void traverse_impl(ptg_graph *g, TravKind kind, uint32_t src, uint32_t *d_value,
                 PTG_CUDA_TRY(cudaGetLastError());
                 PTG_CUDA_TRY(cudaEventRecord(freed, st));
             }
+            if (direct) PTG_CUDA_TRY(cudaStreamWaitEvent(cs, g->direct_done, 0));
             if (link_open) PTG_CUDA_TRY(cudaEventRecord(g->link_ev[1], cs));
         }
         // next frontier: queue from the bitmap; its last CTA ends the level in
@@ -899,9 +991,11 @@ void traverse_impl(ptg_graph *g, TravKind kind, uint32_t src, uint32_t *d_value,
         F = h_ctl->F;
         PTG_REQUIRE(level_error == 0, PTG_ERR_CUDA, "frontier overflow in relax");
         if (link_open) {
-            // the level's copies, first start to last end (the compute stream
-            // waited on every one of them before the sync above)
+            // the level's copies and reads in place, first start to last end (the
+            // compute stream waited on every one of them before the sync
+            // above; the event that follows them on the copy stream is due)
             float lms = 0.f;
+            PTG_CUDA_TRY(cudaEventSynchronize(g->link_ev[1]));
             PTG_CUDA_TRY(cudaEventElapsedTime(&lms, g->link_ev[0], g->link_ev[1]));
             rr.link_ms += lms;
             link_open = false;

@@ -1,0 +1,44 @@
+"""Streamed graphs whose rounds read host memory in place: rows over several
+partitions, sparse and dense rounds, each way the host arrays can lie and each
+placement, against the oracle."""
+import numpy as np
+import pytest
+
+from test_gpu_resident import chain, csr, hubs, random_graph
+
+pytestmark = pytest.mark.gpu
+
+GRAPHS = {
+    "rows_over_partitions": lambda: hubs([1, 16, 129, 1023, 1024, 1025, 9000], 1),
+    "chain": lambda: chain(500, 2),
+    "dense": lambda: random_graph(1999, 300000, 5),
+    "large": lambda: random_graph(100003, 900000, 6),
+}
+
+
+@pytest.mark.parametrize("name", GRAPHS)
+@pytest.mark.parametrize("wide", [False, True])
+@pytest.mark.parametrize("host", ["pinned", "pageable"])
+@pytest.mark.parametrize("policy", ["PREFIX", "NONE", "HOT"])
+def test_streamed_traversals_match_oracle(ptg, ctx, oracle, name, wide, host, policy):
+    torch = pytest.importorskip("torch")
+    n, src, dst, s = GRAPHS[name]()
+    off, col, w = csr(n, src, dst, True, n)
+    keep = None
+    if host == "pinned":
+        keep = [torch.from_numpy(a.view(np.int32)).pin_memory() for a in (col, w)]
+        col, w = [a.numpy().view(np.uint32) for a in keep]
+    m = col.size
+    cfg = ptg.partition_config(partition_bytes=8192, device_budget_bytes=max(3 * 8192, m * 8 // 3), force_out_of_core=1,
+                               hot_threshold=1, resident_policy=getattr(ptg, "PTG_RESIDENT_" + policy))
+    G = ctx.graph(off, col, w, symmetric=False, config=cfg, wide_offsets=wide, pinned=host == "pinned")
+    assert G.info()["out_of_core"] == 1
+    st = {}
+    assert (G.bfs(s, stats=st) == oracle.bfs(off, col, s, method="queue")).all()
+    if name == "chain" and policy == "NONE" and host == "pinned":  # one vertex a round: its edges, not its partition
+        assert st["link_bytes"] <= 4 * m
+    dist = oracle.sssp(off, col, w, s)
+    for delta in (0, 9):
+        assert (G.sssp(s, delta=delta) == dist).all()
+    assert (G.cc() == oracle.cc(off, col)).all()
+    G.close()
