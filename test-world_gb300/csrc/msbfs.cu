@@ -106,15 +106,20 @@ __global__ void __launch_bounds__(kBlock) k_msb_push(const uint32_t *q, const Of
 // Load a vertex's W mask words (16-byte vector loads for W >= 2).
 template <int W>
 __device__ __forceinline__ void load_mask(const u64 *p, u64 (&x)[W]) {
-    if (W == 1) {
+    if constexpr (W == 1) {
         x[0] = p[0];
+    } else if constexpr (W == 2) {
+        const ulonglong2 t = *reinterpret_cast<const ulonglong2 *>(p);
+        x[0] = t.x;
+        x[1] = t.y;
     } else {
-#pragma unroll
-        for (int i = 0; i < W / 2; i++) {
-            ulonglong2 t = reinterpret_cast<const ulonglong2 *>(p)[i];
-            x[2 * i] = t.x;
-            x[2 * i + 1] = t.y;
-        }
+        // one 32-byte load: two of 16 bytes ask L1 for the sector twice, and a
+        // gather of masks is bound by how many it can be asked for
+        static_assert(W == 4);
+        asm volatile("ld.global.v4.b64 {%0, %1, %2, %3}, [%4];"
+                     : "=l"(x[0]), "=l"(x[1]), "=l"(x[2]), "=l"(x[3])
+                     : "l"(p)
+                     : "memory");
     }
 }
 
@@ -183,7 +188,7 @@ struct MsHist {
 // stores: 4.3 GB in 1.0 ms for 256 sources on 4.2 M vertices.  The rows are
 // written once: writing them level by level (a fill, scattered words per
 // level, then a gather to the caller's ids) moved them five times and took
-// 5.7 of that call's 8.8 ms (now 4.7).  Twelve levels are what an RMAT search
+// 5.7 of that call's 8.8 ms (now 3.7).  Twelve levels are what an RMAT search
 // needs (9-10); with eight the second pass over the rows cost another 0.1 ms.
 template <int W, bool FIRST>
 __global__ void __launch_bounds__(kBlock) k_msb_levels(MsHist h, int cnt, uint64_t n, uint32_t k,
@@ -241,7 +246,7 @@ __global__ void __launch_bounds__(kBlock) k_msb_levels(MsHist h, int cnt, uint64
 // adjacency of every other vertex is cut into chunk-edge work items (1024 by
 // default), one warp each (k_msb_pull_big),
 // whose partial masks meet in N through atomicOr.  A neighbour's W words are
-// one 32-byte sector for W = 4, read with 16-byte vector loads.
+// one 32-byte sector for W = 4.
 // Work items (vertex, chunk) of the vertices above `small`; counted first
 // (items == nullptr), then written.  Item order is irrelevant.
 template <class OffT>
@@ -299,8 +304,15 @@ __global__ void __launch_bounds__(kBlock) k_msb_pull_small(uint64_t n, const Off
     }
 }
 
+// What a warp needs before it can gather (an item, its vertex's mask and offsets)
+// is read for kMsbItems items side by side, and the masks meet with the warp's
+// integer reduction.  One item after the other, with shuffles, left a warp
+// waiting for four reads in a row 87% of the time: 256 sources on 4.2 M vertices
+// and 128 M edges 2.27 -> 1.23 ms for the four pull levels (1.37 with 4 items,
+// 1.48 with 16; asking for the next item's columns ahead gave 1%).
+constexpr int kMsbItems = 8;
 template <class OffT, int W>
-__global__ void __launch_bounds__(kBlock) k_msb_pull_big(const uint2 *items, uint64_t nitems, const OffT *off,
+__global__ void __launch_bounds__(kBlock, 4) k_msb_pull_big(const uint2 *items, uint64_t nitems, const OffT *off,
                                                          const uint32_t *col, const u64 *F, const u64 *S, u64 *N,
                                                          const u64 *live_in, uint32_t chunk) {
     constexpr int kU = 4;  // column loads in flight per lane
@@ -309,55 +321,66 @@ __global__ void __launch_bounds__(kBlock) k_msb_pull_big(const uint2 *items, uin
     for (int w = 0; w < W; w++) live[w] = live_in[w];
     const int lane = (int)lane_id();
     const uint64_t nwarps = (uint64_t)gridDim.x * blockDim.x / 32;
-    for (uint64_t it = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) / 32; it < nitems; it += nwarps) {
-        uint2 item = items[it];
-        uint64_t v = item.x;
-        u64 s[W], need[W];
-        load_mask<W>(S + v * W, s);
-        bool none = true;
+    for (uint64_t i0 = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) / 32 * kMsbItems; i0 < nitems; i0 += nwarps * kMsbItems) {
+        // a few items side by side up to their edges: what they need, and where their rows begin
+        uint32_t my_v = 0;
+        OffT my_b = 0, my_e = 0;
+        bool some = false;
+        if (lane < kMsbItems && i0 + lane < nitems) {
+            const uint2 item = items[i0 + lane];
+            my_v = item.x;
+            u64 s[W];
+            load_mask<W>(S + (uint64_t)my_v * W, s);
+            my_b = off[my_v] + (OffT)item.y * (OffT)chunk;
+            my_e = off[(uint64_t)my_v + 1];
+            if (my_e - my_b > (OffT)chunk) my_e = my_b + (OffT)chunk;
 #pragma unroll
-        for (int w = 0; w < W; w++) {
-            need[w] = live[w] & ~s[w];
-            none &= need[w] == 0ull;
+            for (int w = 0; w < W; w++) some |= (live[w] & ~s[w]) != 0ull;
         }
-        if (none) continue;  // warp-uniform: every lane read the same words
-        OffT b = off[v] + (OffT)item.y * (OffT)chunk;
-        OffT e = off[v + 1];
-        if (e - b > (OffT)chunk) e = b + (OffT)chunk;
-        u64 acc[W];
+        unsigned todo = __ballot_sync(0xffffffffu, some);
+        while (todo) {
+            const int from = __ffs(todo) - 1;
+            todo &= todo - 1;
+            const uint64_t v = __shfl_sync(0xffffffffu, my_v, from);
+            const OffT b = __shfl_sync(0xffffffffu, my_b, from), e = __shfl_sync(0xffffffffu, my_e, from);
+            u64 s[W], need[W];
+            load_mask<W>(S + v * W, s);
 #pragma unroll
-        for (int w = 0; w < W; w++) acc[w] = 0;
-        for (OffT k0 = b; k0 < e; k0 += 32 * kU) {
-            uint32_t c[kU];
+            for (int w = 0; w < W; w++) need[w] = live[w] & ~s[w];
+            u64 acc[W];
 #pragma unroll
-            for (int j = 0; j < kU; j++) {
-                OffT k = k0 + (OffT)(j * 32 + lane);
-                c[j] = k < e ? col[k] : 0u;
-            }
+            for (int w = 0; w < W; w++) acc[w] = 0;
+            for (OffT k0 = b; k0 < e; k0 += 32 * kU) {
+                uint32_t c[kU];
 #pragma unroll
-            for (int j = 0; j < kU; j++) {
-                if (k0 + (OffT)(j * 32 + lane) < e) {
-                    u64 f[W];
-                    load_mask<W>(F + (uint64_t)c[j] * W, f);
-#pragma unroll
-                    for (int w = 0; w < W; w++) acc[w] |= f[w];
+                for (int j = 0; j < kU; j++) {
+                    OffT k = k0 + (OffT)(j * 32 + lane);
+                    c[j] = k < e ? col[k] : 0u;
                 }
+#pragma unroll
+                for (int j = 0; j < kU; j++) {
+                    if (k0 + (OffT)(j * 32 + lane) < e) {
+                        u64 f[W];
+                        load_mask<W>(F + (uint64_t)c[j] * W, f);
+#pragma unroll
+                        for (int w = 0; w < W; w++) acc[w] |= f[w];
+                    }
+                }
+                bool done = true;
+#pragma unroll
+                for (int w = 0; w < W; w++) {
+                    const u64 x = (u64)__reduce_or_sync(0xffffffffu, (unsigned)(acc[w] >> 32)) << 32 |
+                                  __reduce_or_sync(0xffffffffu, (unsigned)acc[w]);
+                    acc[w] = x;
+                    done &= (x & need[w]) == need[w];
+                }
+                if (done) break;  // warp-uniform after the all-reduce
             }
-            bool done = true;
 #pragma unroll
             for (int w = 0; w < W; w++) {
-                u64 x = acc[w];
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) x |= __shfl_xor_sync(0xffffffffu, x, o);
-                acc[w] = x;
-                done &= (x & need[w]) == need[w];
+                u64 x = acc[w] & need[w];
+                if (lane == w && x) atomicOr(&N[v * W + w], x);
             }
-            if (done) break;  // warp-uniform after the all-reduce
-        }
-#pragma unroll
-        for (int w = 0; w < W; w++) {
-            u64 x = acc[w] & need[w];
-            if (lane == w && x) atomicOr(&N[v * W + w], x);
         }
     }
 }
