@@ -528,36 +528,51 @@ __global__ void __launch_bounds__(kBlock) k_mss_relax(const uint32_t *q, const O
 // neighbours in registers and writes its own distances once.  Pushing the same
 // round sends two reductions of 8 sectors per edge to L2 and takes three times
 // the instructions per edge: 2.4 and 2.1 ms in the two heaviest rounds of 64
-// sources on RMAT-20, 0.9 ms a round on average here.  Work is split as in the MS-BFS pull:
+// sources on RMAT-20, 0.52 ms a round on average here.  Work is split as in the MS-BFS pull:
 // rows of up to `small` edges by 32-vertex groups, longer ones in chunks, a
 // warp each; 32 edges are loaded side by side, those that pass the bound of
-// k_mss_queue are taken 8 at a time by the whole warp.  A row in several
+// k_mss_queue are taken 8 at a time by the whole warp, all 64 sources alike:
+// where a source is not active its candidate was offered before and improves
+// nothing, and a test would cost as much as the candidate.  A row in several
 // chunks meets in atomics.  Distances read may be this round's already (they
 // only fall, and an improved vertex is queued for the next round).
 struct MssEdge {
-    uint32_t u, w, lo, hi;  // neighbour, weight, its active sources
+    uint32_t u, w;  // neighbour and weight
 };
 
 template <class OffT>
 __device__ __forceinline__ void mss_pull_row(OffT b, OffT e, uint64_t v, bool alone, const uint32_t *col,
                                              const uint32_t *w, uint32_t *dist, const u64 *A, u64 *N,
                                              const int *dmin, int top, MssEdge *pass) {
-    const unsigned lane = lane_id(), bit = 1u << lane;
+    const unsigned lane = lane_id();
     bool loaded = false;
     uint2 own = make_uint2(0u, 0u), best = own;
+    // the next 32 edges, and what says whether they pass, are on their way
+    // while the present ones are taken (one step after the other: 7.0 instead
+    // of 5.1 ms for the eight pull rounds of 128 sources on RMAT-20; rows side
+    // by side as in k_msb_pull_big need more registers and gave that back)
+    bool ok = b + (OffT)lane < e;
+    uint32_t ul = ok ? __ldcs(col + b + lane) : 0u, wl = ok ? __ldcs(w + b + lane) : 0u;
+    bool some = ok && A[ul] != 0ull;
+    int least = ok ? dmin[ul] : 0;
     for (OffT k0 = b; k0 < e; k0 += 32) {
-        const bool ok = k0 + (OffT)lane < e;
-        const uint32_t ul = ok ? __ldcs(col + k0 + lane) : 0u, wl = ok ? __ldcs(w + k0 + lane) : 0u;
-        const u64 al = ok ? A[ul] : 0ull;
-        const bool keep = al != 0 && (top >= kMssNone || (long long)dmin[ul] + wl < top);
+        const OffT kn = k0 + 32 + (OffT)lane;
+        const bool okn = kn < e;
+        const uint32_t un = okn ? __ldcs(col + kn) : 0u, wn = okn ? __ldcs(w + kn) : 0u;
+        const bool keep = some && (top >= kMssNone || (long long)least + wl < top);
+        const uint32_t uk = ul, wk = wl;
+        ul = un;
+        wl = wn;
+        some = okn && A[un] != 0ull;
+        least = okn ? dmin[un] : 0;
         const unsigned left = __ballot_sync(0xffffffffu, keep);
         if (!left) continue;
         // the edges that pass, side by side in shared memory, padded with
-        // edges that no source is active at (reading them back broadcast takes
-        // one instruction where shuffles took nine)
+        // the vertex itself (reading them back broadcast takes one instruction
+        // where shuffles took nine)
         const int cnt = __popc(left), at = keep ? __popc(left & lanemask_lt()) : cnt + __popc(~left & lanemask_lt());
         __syncwarp();
-        pass[at] = MssEdge{keep ? ul : (uint32_t)v, wl, keep ? (uint32_t)al : 0u, keep ? (uint32_t)(al >> 32) : 0u};
+        pass[at] = MssEdge{keep ? uk : (uint32_t)v, keep ? wk : 0u};
         __syncwarp();
         if (!loaded) {
             own = reinterpret_cast<const uint2 *>(dist + v * 64)[lane];
@@ -571,9 +586,9 @@ __device__ __forceinline__ void mss_pull_row(OffT b, OffT e, uint64_t v, bool al
             for (int t = 0; t < kN; t++) d[t] = reinterpret_cast<const uint2 *>(dist + (uint64_t)pass[i + t].u * 64)[lane];
 #pragma unroll
             for (int t = 0; t < kN; t++) {
-                const MssEdge x = pass[i + t];
-                if (x.lo & bit) best.x = min(best.x, d[t].x + x.w);
-                if (x.hi & bit) best.y = min(best.y, d[t].y + x.w);
+                const uint32_t add = pass[i + t].w;
+                best.x = __viaddmin_u32(min(d[t].x, ~add), add, best.x);
+                best.y = __viaddmin_u32(min(d[t].y, ~add), add, best.y);
             }
         };
         int i = 0;
@@ -716,21 +731,35 @@ __global__ void __launch_bounds__(kBlock) k_mss_queue(const u64 *M, uint64_t n, 
     if (threadIdx.x == 0 && degsum) atomicAdd(&ctl->m_unvisited, degsum);
 }
 
-// dist[x*64 + s] -> out[s*n + v] for s < k (32 vertices x 64 sources per
-// tile), x = newid[v] on a regrouped graph (else v).
+// dist[x*64 + s] -> out[s*n + v] for s < k, x = newid[v] on a regrouped graph
+// (else v).  Tiles of 64 vertices x 64 sources; a warp has 8 vertices' rows in
+// flight and writes 256 bytes of a result row.  (With 32 vertices, an element
+// of one row at a time per thread: 250 us for 64 sources on 1 M vertices, now
+// 85; 0.5 GB moved.)
+constexpr int kTrVerts = 64;
 __global__ void __launch_bounds__(kBlock) k_mss_transpose(const uint32_t *dist, uint64_t n, uint32_t k,
                                                           const uint32_t *newid, uint32_t *out) {
-    __shared__ uint32_t t[32][65];
-    for (uint64_t v0 = (uint64_t)blockIdx.x * 32; v0 < n; v0 += (uint64_t)gridDim.x * 32) {
-        for (int i = threadIdx.x; i < 32 * 64; i += kBlock) {
-            int vv = i / 64, s = i % 64;
-            uint64_t x = v0 + vv < n ? (newid ? (uint64_t)newid[v0 + vv] : v0 + vv) : 0;
-            t[vv][s] = v0 + vv < n ? dist[x * 64 + s] : 0u;
+    constexpr int kEach = kTrVerts / (kBlock / 32);
+    __shared__ uint32_t t[kTrVerts][65];
+    const unsigned lane = lane_id(), wid = threadIdx.x >> 5;
+    for (uint64_t v0 = (uint64_t)blockIdx.x * kTrVerts; v0 < n; v0 += (uint64_t)gridDim.x * kTrVerts) {
+        const uint64_t mine = min(v0 + wid * kEach + lane % kEach, n - 1);
+        const uint32_t x = newid ? newid[mine] : (uint32_t)mine;
+        uint2 d[kEach];
+#pragma unroll
+        for (int i = 0; i < kEach; i++)
+            d[i] = __ldcs(reinterpret_cast<const uint2 *>(dist + (uint64_t)__shfl_sync(0xffffffffu, x, i) * 64) + lane);
+#pragma unroll
+        for (int i = 0; i < kEach; i++) {
+            t[wid * kEach + i][2 * lane] = d[i].x;
+            t[wid * kEach + i][2 * lane + 1] = d[i].y;
         }
         __syncthreads();
-        for (int i = threadIdx.x; i < 32 * 64; i += kBlock) {
-            int s = i / 32, vv = i % 32;
-            if (s < (int)k && v0 + vv < n) out[(uint64_t)s * n + v0 + vv] = t[vv][s];
+        for (uint32_t s = wid; s < k; s += kBlock / 32) {
+            uint32_t *row = out + (uint64_t)s * n + v0;
+#pragma unroll
+            for (int j = 0; j < kTrVerts; j += 32)
+                if (v0 + j + lane < n) __stcs(row + j + lane, t[j + lane][s]);
         }
         __syncthreads();
     }
@@ -953,7 +982,7 @@ void msbfs_impl(ptg_graph *g, const uint32_t *h_srcs, uint32_t k, uint32_t *d_ro
             launch(ctx, "k_msb_pull_small", k_msb_pull_small<OffT, W>, vgrid, kBlock, 0, st, n, off, col,
                    Mc, (const u64 *)S, Mn, (const u64 *)d_live[round], g->pull_small);
             if (g->n_pull_items)
-                launch(ctx, "k_msb_pull_big", k_msb_pull_big<OffT, W>, sms * 8, kBlock, 0, st,
+                launch(ctx, "k_msb_pull_big", k_msb_pull_big<OffT, W>, sms * 32, kBlock, 0, st,
                        (const uint2 *)g->d_pull_items.p, g->n_pull_items, off, col, Mc,
                        (const u64 *)S, Mn, (const u64 *)d_live[round], g->pull_chunk);
         } else {
@@ -1038,10 +1067,12 @@ void mssssp_impl(ptg_graph *g, const uint32_t *h_srcs, uint32_t k, uint32_t *d_r
         rr.iterations++;
         u64 *Mc = cur ? M1 : M0, *Mn = cur ? M0 : M1;
         PTG_CUDA_TRY(cudaMemsetAsync(Mn, 0, n * 8, st));
-        const bool pull = can_pull && Eact * 2 > m;
+        // 64 sources on RMAT-20, two batches: 7.4 ms with the line at m / 5, 8.0 at
+        // m / 2 and 7.6 at m / 16 (a pull round reads every edge's filter)
+        const bool pull = can_pull && Eact * 5 > m;
         const uint64_t scanned = Eact;
         if (pull) {
-            launch(ctx, "k_mss_pull", k_mss_pull<OffT>, sms * 8, kBlock, 0, st, (const uint2 *)g->d_pull_items.p,
+            launch(ctx, "k_mss_pull", k_mss_pull<OffT>, sms * 40, kBlock, 0, st, (const uint2 *)g->d_pull_items.p,
                    g->n_pull_items, g->pull_small, g->pull_chunk, n, off, col, wt, dist, (const u64 *)Mc, Mn,
                    (const int *)dmin, (const int *)dmax);
         } else {
@@ -1057,7 +1088,7 @@ void mssssp_impl(ptg_graph *g, const uint32_t *h_srcs, uint32_t k, uint32_t *d_r
         rr.edges_relaxed += pull ? scanned : E;
         cur ^= 1;
     }
-    launch(ctx, "k_mss_transpose", k_mss_transpose, grid_for((n + 31) / 32, 1, sms * 8), kBlock, 0, st,
+    launch(ctx, "k_mss_transpose", k_mss_transpose, grid_for(n, kTrVerts, sms * 8), kBlock, 0, st,
            (const uint32_t *)dist, n, k, (const uint32_t *)(g->relabeled ? g->d_newid.p : nullptr), d_rows);
     PTG_CUDA_TRY(cudaGetLastError());
 }
