@@ -2,9 +2,9 @@
 //
 // ptg_msbfs / ptg_mssssp take k sources and fill k rows of results, each row
 // equal to a single-source ptg_bfs / ptg_sssp call.  Sources are processed in
-// groups of 64 (one 64-bit mask word per vertex, msbfs.cu); host outputs are
-// produced group by group in a device buffer of 64 rows and copied out while
-// the next group runs.  Graphs the fused kernels do not cover (out-of-core)
+// groups (up to 256 BFS or 64 SSSP sources, msbfs.cu); host outputs are
+// produced group by group in a device buffer of that many rows and copied out
+// while the next group runs.  Graphs the fused kernels do not cover (out-of-core)
 // run the single-source traversal row by row.
 #include <algorithm>
 #include <cstring>

@@ -11,13 +11,15 @@
 //   frontier's edges like the single-source expand) or, when the frontier's
 //   edges are a large share of the graph and the graph is symmetric, pulls
 //   (every vertex ORs its neighbours' F, stopping once all sources saw it).
-//   With W = 4 one 32-byte sector read per edge serves 256 sources.
+//   With W = 4 one 32-byte sector read per edge serves 256 sources.  The
+//   levels' frontier masks are kept, and the result rows written from them once.
 // MS-SSSP: distances stored vertex-major, dist[v*64 + s], so the 64 distances
 //   of a vertex are two 128-byte lines; a warp relaxes one edge for 64
-//   sources at once (lane l handles sources l and l+32), only for sources
-//   whose distance at the edge's tail improved in the previous round (a
-//   64-bit active mask per vertex); improvements set bits of the target's
-//   next mask with one reduction per edge.  Rounds run until no mask is set.
+//   sources at once (lane l handles sources 2l and 2l+1).  A vertex is active
+//   while some source improved it in the previous round (a 64-bit mask);
+//   an edge is looked at only if bounds on all 64 distances of its ends let it
+//   improve one (k_mss_queue).  Rounds push, or pull when many edges are active
+//   and weights are the same both ways, until no mask is set.
 // Results equal k single-source calls (tests compare them row by row).
 #include <algorithm>
 #include <climits>
@@ -188,7 +190,7 @@ struct MsHist {
 // stores: 4.3 GB in 1.0 ms for 256 sources on 4.2 M vertices.  The rows are
 // written once: writing them level by level (a fill, scattered words per
 // level, then a gather to the caller's ids) moved them five times and took
-// 5.7 of that call's 8.8 ms (now 3.7).  Twelve levels are what an RMAT search
+// 5.7 of that call's 8.8 ms (now 3.6).  Twelve levels are what an RMAT search
 // needs (9-10); with eight the second pass over the rows cost another 0.1 ms.
 template <int W, bool FIRST>
 __global__ void __launch_bounds__(kBlock) k_msb_levels(MsHist h, int cnt, uint64_t n, uint32_t k,

@@ -48,8 +48,9 @@
 // about what PageRank's gathers reach from L2 (one 32-byte sector each): the
 // round of 307 M edges took 1170 us as a push and takes 730 as a pull.  Staging the edges ahead with cp.async and dropping candidates by the largest
 // distance among the hubs changed neither.  Per search, before -> now: BFS on
-// RMAT-16 217 -> 87 us, on RMAT-24 580 -> 415 us; SSSP on RMAT-24 6.7 -> 3.5
-// ms; a served mix of small graphs 8.8 -> 6.5 ms.
+// RMAT-16 217 -> 87 us, on RMAT-24 580 -> 415 us; SSSP on RMAT-24 6.7 -> 3.2
+// ms; a served mix of small graphs 8.8 -> 6.5 ms (5.5 with PageRank's one launch
+// per iteration).
 #include <algorithm>
 #include <cmath>
 #include <cstring>

@@ -39,7 +39,7 @@
 //    CPU threads gather active adjacency into a unified-memory buffer the GPU
 //    page-faults on, main.cu:1126-1156, 1336-1378).  The count is on the host
 //    while the resident edges are relaxed, so copies start meanwhile.  SSSP of
-//    a directed RMAT-22 with half of its edges streamed: 12.2 -> 5.9 ms.
+//    a directed RMAT-22 with half of its edges streamed: 11.6 -> 4.8 ms.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
