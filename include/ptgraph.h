@@ -156,7 +156,7 @@ enum {
 
 typedef struct ptg_run_stats {
     uint32_t iterations;        /* frontier rounds (BFS levels, SSSP rounds, ...)  */
-    uint32_t bottom_up_rounds;  /* BFS rounds run bottom-up                        */
+    uint32_t bottom_up_rounds;  /* BFS and SSSP rounds run as a pull               */
     uint64_t edges_relaxed;     /* edges inspected by relax kernels                */
     uint64_t vertices_reached;  /* vertices with a finite value                    */
     uint64_t edges_in_component;/* directed edges out of reached vertices          */
