@@ -876,6 +876,7 @@ void traverse_impl(ptg_graph *g, TravKind kind, uint32_t src, uint32_t *d_value,
             // 6.2, 4.9, 4.8, 4.8, 5.2 ms; RMAT-24 all streamed 55, 26.6, 21.9,
             // 21.4, 21.4, 23.3 ms; BFS of the former 4.5, 2.0, 1.9, 1.9, 1.9, 1.9.
             uint64_t active = 0, direct = 0;  // streamed edges of the frontier; those read in place
+            uint64_t spared = 0;              // edges that are not copied for that
             for (uint64_t p = g->resident_partitions; p < P && hot; p++) g->part_visits[p] += h_hits[p];
             for (uint64_t p = g->resident_partitions; p < P; p++) {
                 const uint64_t e0 = p * g->partition_edges, e1 = std::min<uint64_t>(g->m, e0 + g->partition_edges);
@@ -886,9 +887,16 @@ void traverse_impl(ptg_graph *g, TravKind kind, uint32_t src, uint32_t *d_value,
                 active += h_hits[p];
                 if (h_direct[p]) {
                     direct += h_hits[p];
-                    rr.parts_streamed++;
+                    spared += e1 - e0 - h_hits[p];
                 }
             }
+            // the kernel walks the other partitions' active edges too, more than
+            // four times as fast as the link would bring the spared ones
+            if (spared * 4 < active) {
+                std::memset(h_direct + g->resident_partitions, 0, P - g->resident_partitions);
+                direct = 0;
+            }
+            for (uint64_t p = g->resident_partitions; p < P; p++) rr.parts_streamed += h_direct[p];
             if (direct) {
                 ws.tiles.ensure((active / kTile + 4) * sizeof(uint32_t));
                 tr = ws.tiles.as<uint32_t>();
