@@ -78,6 +78,22 @@ constexpr u64 kWideEdges = 1ull << 21;
 // polls of the barrier before a CTA gives up (tens of seconds)
 constexpr u64 kBarrierPolls = 1ull << 26;
 
+// Every thread takes the launch's decisions for itself, from words that it reads
+// after a barrier.  A thread may be late with that read (another lane's kernels on
+// its SM, a context switch), while others are on their way to the next barrier
+// already, so no word that decides is written between the barrier before its read
+// and the one after:
+//   found, edges, few, items, bigs, least  the frontier's, by level % 3: a level reads
+//       its own, adds to the next one's and clears the one after that, whose last
+//       reader was the level before.  A bucket pass of SSSP fills the lists of the
+//       present level (their tails and `least` are read by the round behind its
+//       barrier only), but what it found it counts elsewhere:
+//   bucket_found, bucket_edges, far_min    by pass % 3: a pass adds to its own, reads
+//       those of the pass before and clears the next one's
+//   cands                                  by level % 4: read by the next level, cleared
+//       three levels on
+//   pull_edges, pull_items, pull_bigs      by heavy round % 2: cleared behind the barrier
+//       that the following heavy round counts up to
 struct ResCtl {
     unsigned arrive, gen;           // grid barrier
     unsigned error;
@@ -85,6 +101,7 @@ struct ResCtl {
     // kSmallDeg, and longer ones << 32 | their pieces
     u64 few[3], items[3], bigs[3];
     u64 found[3], edges[3];         // the frontier's vertices and edges
+    u64 bucket_found[3], bucket_edges[3];  // SSSP: those that a bucket pass took, by turn
     u64 far_min[3];                 // SSSP: least distance that stays parked, by turn
     u64 cands[4];                   // unvisited vertices that a pull round looked at (level % 4)
     unsigned chunk[2];              // pull work counter, by level parity
@@ -704,7 +721,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_traverse(ResArgs a) {
     }
     if (leader) {
         for (int i = 0; i < 3; i++) ctl->few[i] = ctl->items[i] = ctl->bigs[i] = ctl->found[i] = ctl->edges[i] = 0;
-        for (int i = 0; i < 3; i++) ctl->far_min[i] = ~0ull;
+        for (int i = 0; i < 3; i++) ctl->far_min[i] = ~0ull, ctl->bucket_found[i] = ctl->bucket_edges[i] = 0;
         ctl->chunk[0] = ctl->chunk[1] = 0;
         for (int i = 0; i < 4; i++) ctl->cands[i] = 0;
         for (int i = 0; i < 3; i++) ctl->least[i] = PTG_UNREACHED;
@@ -748,7 +765,9 @@ __global__ void __launch_bounds__(kBlock, 4) k_traverse(ResArgs a) {
     int cur = 0;
     while (true) {
         const int slot = level % 3, next = (level + 1) % 3, later = (level + 2) % 3;
-        u64 F = ctl->found[slot], E = ctl->edges[slot];
+        // (after a bucket pass: what it took, the round before had found nothing)
+        u64 F = scanned ? ctl->bucket_found[(far_turn + 2) % 3] : ctl->found[slot];
+        u64 E = scanned ? ctl->bucket_edges[(far_turn + 2) % 3] : ctl->edges[slot];
         const Frontier front = frontier_of(a, cur, slot);
         if (MODE == 2 && level == 0) F = a.n, E = a.m;
         if (F == 0) {
@@ -769,7 +788,11 @@ __global__ void __launch_bounds__(kBlock, 4) k_traverse(ResArgs a) {
             }
             scanned = true;
             const uint32_t to = from + delta >= PTG_UNREACHED ? PTG_UNREACHED : (uint32_t)(from + delta);
-            if (leader) ctl->far_min[(far_turn + 1) % 3] = ~0ull;
+            if (leader) {
+                const int after = (far_turn + 1) % 3;
+                ctl->far_min[after] = ~0ull;
+                ctl->bucket_found[after] = ctl->bucket_edges[after] = 0;
+            }
             uint32_t best = PTG_UNREACHED;
             for (uint64_t w0 = (tid >> 5) * 32; w0 < words; w0 += nthreads) {
                 const uint64_t wd = w0 + lane_id();
@@ -800,7 +823,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_traverse(ResArgs a) {
             }
             best = __reduce_min_sync(0xffffffffu, best);
             if (lane_id() == 0 && best != PTG_UNREACHED) atomicMin(&ctl->far_min[far_turn % 3], (u64)best);
-            buf_finish<OffT>(buf, a, front, &ctl->found[slot], &ctl->edges[slot]);
+            buf_finish<OffT>(buf, a, front, &ctl->bucket_found[far_turn % 3], &ctl->bucket_edges[far_turn % 3]);
             thr = to;
             far_turn++;
             if (!grid_barrier(ctl)) return;

@@ -135,3 +135,39 @@ def test_sssp_pull_rounds(ptg, ctx, ctx_grouped, oracle, grouped, wide, both_way
         assert (G.sssp(s, delta=delta, flags=ptg.PTG_NO_DIRECTION_OPT, stats=st) == dist).all(), delta
         assert st["bottom_up_rounds"] == 0
     G.close()
+
+
+def test_buckets_beside_another_search(ptg, ctx, oracle):
+    """Narrow buckets (a pass over the parked vertices per round or two) while another context's
+    searches hold the same SMs, so that CTAs leave a barrier at very different times."""
+    import threading
+    cases = []
+    for name in ("edge_degrees", "chain", "sparse", "large"):
+        n, src, dst, s = GRAPHS[name]()
+        off, col, w = csr(n, src, dst, True, n)
+        cases.append((off, col, w, s, oracle.sssp(off, col, w, s)))
+    other = ptg.Ctx(0)
+    wrong, stop = [], threading.Event()
+
+    def search(c, rounds):
+        try:
+            graphs = [c.graph(off, col, w, symmetric=True) for off, col, w, _, _ in cases]
+            for r in range(rounds):
+                if stop.is_set():
+                    break
+                for i, (g, case) in enumerate(zip(graphs, cases)):
+                    for delta in (1, 7):
+                        if not (g.sssp(case[3], delta=delta) == case[4]).all():
+                            wrong.append((i, delta, r))
+            for g in graphs:
+                g.close()
+        except Exception as e:
+            wrong.append(repr(e))
+
+    t = threading.Thread(target=search, args=(other, 1000))
+    t.start()
+    search(ctx, 10)
+    stop.set()
+    t.join()
+    other.close()
+    assert not wrong, wrong
