@@ -24,6 +24,12 @@ inline int grid_for(uint64_t work, int per_block, int max_blocks) {
     return (int)b;
 }
 
+// End of the SSSP bucket that begins at distance `from`: a width that reaches the
+// value of an unreached vertex (callers may ask for any) takes all the rest.
+__host__ __device__ inline uint32_t bucket_end(uint64_t from, uint64_t width) {
+    return from + width >= PTG_UNREACHED ? PTG_UNREACHED : (uint32_t)(from + width);
+}
+
 __device__ __forceinline__ unsigned lane_id() { return threadIdx.x & 31u; }
 
 __device__ __forceinline__ unsigned lanemask_lt() {

@@ -760,7 +760,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_traverse(ResArgs a) {
     uint32_t iterations = 0, pulls = 0, level = 0, far_turn = 0, pull_turn = 0, late_pulls = 0;
     uint32_t thr = PTG_UNREACHED;
     u64 delta = a.delta, bucket_E = 0;
-    if (MODE == 1 && a.use_far) thr = a.base + a.delta;
+    if (MODE == 1 && a.use_far) thr = bucket_end(a.base, a.delta);
     bool bottom_up = false, limit = false, scanned = false;
     int cur = 0;
     while (true) {
@@ -787,7 +787,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_traverse(ResArgs a) {
                 bucket_E = 0;
             }
             scanned = true;
-            const uint32_t to = from + delta >= PTG_UNREACHED ? PTG_UNREACHED : (uint32_t)(from + delta);
+            const uint32_t to = bucket_end(from, delta);
             if (leader) {
                 const int after = (far_turn + 1) % 3;
                 ctl->far_min[after] = ~0ull;
@@ -810,7 +810,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_traverse(ResArgs a) {
                         d[j] = (bits[j] >> lane_id()) & 1u ? a.value[(w0 + i + j) * 32 + lane_id()] : 0u;
 #pragma unroll
                     for (int j = 0; j < 4; j++) {
-                        const bool near = d[j] >= thr && d[j] < to;
+                        const bool near = ((bits[j] >> lane_id()) & 1u) && d[j] >= thr && d[j] < to;
                         if (near) buf.least = min(buf.least, d[j]);
                         else if (d[j] >= thr) best = min(best, d[j]);
                         buf_add(buf, near, (uint32_t)((w0 + i + j) * 32 + lane_id()));

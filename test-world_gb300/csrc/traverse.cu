@@ -778,7 +778,7 @@ void traverse_impl(ptg_graph *g, TravKind kind, uint32_t src, uint32_t *d_value,
         launch(ctx, "k_fill_u32", k_fill_u32, fill_grid, kBlock, 0, st, d_value, n, PTG_UNREACHED);
         init.F = 1;
         if (use_far) {
-            init.threshold = base + delta;
+            init.threshold = bucket_end(base, delta);
             PTG_CUDA_TRY(cudaMemsetAsync(ws.farbm.p, 0, words * 4, st));
         }
     }
@@ -818,8 +818,7 @@ void traverse_impl(ptg_graph *g, TravKind kind, uint32_t src, uint32_t *d_value,
             PTG_CUDA_TRY(cudaMemcpyAsync(h_ctl, d_ctl, sizeof(TravCtl), cudaMemcpyDeviceToHost, st));
             PTG_CUDA_TRY(cudaStreamSynchronize(st));
             if (h_ctl->far_min == ~0ull) break;  // far pile empty
-            uint64_t thr64 = h_ctl->far_min + delta;
-            threshold = thr64 >= PTG_UNREACHED ? PTG_UNREACHED : (uint32_t)thr64;
+            threshold = bucket_end(h_ctl->far_min, delta);
             TravCtl upd = *h_ctl;
             upd.threshold = threshold;
             upd.next_tail = 0;

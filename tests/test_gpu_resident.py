@@ -171,3 +171,20 @@ def test_buckets_beside_another_search(ptg, ctx, oracle):
     t.join()
     other.close()
     assert not wrong, wrong
+
+
+@pytest.mark.parametrize("delta", [0xFFFFFFFD, 0xFFFFFFFE, 0xFFFFFFFF])
+@pytest.mark.parametrize("zero_based", [False, True])
+@pytest.mark.parametrize("name", ["edge_degrees", "sparse", "one_cta"])
+@pytest.mark.parametrize("streamed", [False, True])
+def test_bucket_width_past_every_distance(ptg, ctx, oracle, name, delta, zero_based, streamed):
+    """Widths whose sum with the source's value reaches or passes 2^32: one bucket holds everything."""
+    n, src, dst, s = GRAPHS[name]()
+    off, col, w = csr(n, src, dst, not streamed, n)
+    cfg = ptg.partition_config(partition_bytes=1024, device_budget_bytes=4096, force_out_of_core=1) if streamed else None
+    G = ctx.graph(off, col, w, symmetric=not streamed, config=cfg)
+    assert G.info()["out_of_core"] == int(streamed)
+    dist = oracle.sssp(off, col, w, s)
+    want = np.where(dist == 0xFFFFFFFF, dist, dist - 1) if zero_based else dist
+    assert (G.sssp(s, delta=delta, flags=ptg.PTG_LEVEL_ZERO_BASED if zero_based else 0) == want).all()
+    G.close()
