@@ -638,30 +638,55 @@ __global__ void __launch_bounds__(kBlock) k_far_split(uint32_t *far_bm, uint64_t
     }
 }
 
+// Whether a kernel may read the edges [e0, e1) in host memory.
+bool readable_in_place(const ptg_graph *g, uint64_t e0, uint64_t e1, bool weights) {
+    auto in = [&](int which, const uint32_t *h, const uint32_t *d) {
+        return d && (uintptr_t)(h + e0) >= g->pin_lo[which] && (uintptr_t)(h + e1) <= g->pin_hi[which];
+    };
+    return in(0, g->h_col, g->dev_col) && (!weights || in(1, g->h_w, g->dev_w));
+}
+
 // Hot-partition cache (the reference's visit-counted fragment promotion,
 // gpu_kernels.cu:254-282 and 475-485, where a 4096-edge fragment whose visit
 // record exceeds 3600 becomes a swap candidate).  part_visits[p] accumulates
 // the edges of frontier vertices that fell in partition p; a partition is hot
 // once that exceeds hot_threshold visits per 4096 edges.  A hot partition
-// takes a free slot, or the slot of the coldest cached partition if that one
-// has fewer visits; a cached partition is relaxed from its slot without a
-// copy, in this and every later traversal of the graph.  Returns the slot,
-// or -1 to use a staging buffer.
-int hot_victim(const ptg_graph *g, uint64_t p, uint64_t edges) {
+// takes a free slot, or the slot of the least worthy cached partition if it is
+// worthier itself; a cached partition is relaxed from its slot without a
+// copy, in this and every later traversal of the graph.
+//
+// A partition that kernels cannot read in place (the pages at the ends of the
+// caller's arrays are not page-locked) is copied whole for a single active
+// edge, so it is worthier than any that they can; else visits decide.
+bool less_worthy(const ptg_graph *g, uint64_t a, uint64_t b) {
+    auto in_place = [&](uint64_t p) {
+        const uint64_t e0 = p * g->partition_edges;
+        return readable_in_place(g, e0, std::min(g->m, e0 + g->partition_edges), g->weighted);
+    };
+    const bool ra = in_place(a), rb = in_place(b);
+    return ra != rb ? ra : g->part_visits[a] < g->part_visits[b];
+}
+
+// The slot that hot partition p may take in a round with these active edges per
+// partition, -1 if none: not one whose partition the round has yet to use.
+int hot_victim(const ptg_graph *g, uint64_t p, uint64_t edges, const unsigned long long *hits) {
     if (g->cache_static) return -1;
     if ((double)g->part_visits[p] * 4096.0 <= (double)g->hot_threshold * (double)edges) return -1;
     int victim = -1;
     for (uint32_t s = 0; s < g->cache_slots; s++) {
-        int64_t q = g->slots[s].part;
+        const int64_t q = g->slots[s].part;
         if (q < 0) return (int)s;
-        if (victim < 0 || g->part_visits[q] < g->part_visits[g->slots[victim].part]) victim = (int)s;
+        if (hits[q] && (uint64_t)q > p) continue;
+        if (victim < 0 || less_worthy(g, q, g->slots[victim].part)) victim = (int)s;
     }
-    return victim >= 0 && g->part_visits[g->slots[victim].part] < g->part_visits[p] ? victim : -1;
+    return victim >= 0 && less_worthy(g, g->slots[victim].part, p) ? victim : -1;
 }
 
-int hot_slot(ptg_graph *g, uint64_t p, uint64_t edges) {
+// The slot of a partition that is copied now: its own, or one that it takes; -1
+// to use a staging buffer.
+int hot_slot(ptg_graph *g, uint64_t p, uint64_t edges, const unsigned long long *hits) {
     if (g->slot_of[p] >= 0) return g->slot_of[p];
-    const int victim = hot_victim(g, p, edges);
+    const int victim = hot_victim(g, p, edges, hits);
     if (victim < 0) return -1;
     HotSlot &hs = g->slots[victim];
     if (hs.part >= 0) g->slot_of[hs.part] = -1;
@@ -674,17 +699,24 @@ int hot_slot(ptg_graph *g, uint64_t p, uint64_t edges) {
     return victim;
 }
 
+// Whether partition p, of which a round reads few edges (they would be read in
+// place), is in a cache slot or takes one now.  A hot partition's edges were about
+// all read over the link by then, and it is copied once to end that: into a
+// free slot, or one whose partition this round does not use and that was visited
+// less than half as often (copying costs more than reading in place, so two
+// partitions of about the same use must not take a slot from each other in turn).
+bool sparse_slot(ptg_graph *g, uint64_t p, uint64_t edges, const unsigned long long *hits) {
+    if (g->slot_of[p] >= 0) return true;
+    const int victim = hot_victim(g, p, edges, hits);
+    if (victim < 0) return false;
+    const int64_t q = g->slots[victim].part;
+    if (q >= 0 && (hits[q] || g->part_visits[q] * 2 >= g->part_visits[p])) return false;
+    return hot_slot(g, p, edges, hits) >= 0;
+}
+
 // ---------------------------------------------------------------------------
 // host driver
 // ---------------------------------------------------------------------------
-// Whether a kernel may read the edges [e0, e1) in host memory.
-bool readable_in_place(const ptg_graph *g, uint64_t e0, uint64_t e1, bool weights) {
-    auto in = [&](int which, const uint32_t *h, const uint32_t *d) {
-        return d && (uintptr_t)(h + e0) >= g->pin_lo[which] && (uintptr_t)(h + e1) <= g->pin_hi[which];
-    };
-    return in(0, g->h_col, g->dev_col) && (!weights || in(1, g->h_w, g->dev_w));
-}
-
 // Scan of the frontier's degrees, of the edges in [from, to) only: prefix sums
 // and row starts in ws.scan / ws.rowstart, and the row that every tile begins in.
 template <class OffT>
@@ -880,8 +912,8 @@ void traverse_impl(ptg_graph *g, TravKind kind, uint32_t src, uint32_t *d_value,
             for (uint64_t p = g->resident_partitions; p < P; p++) {
                 const uint64_t e0 = p * g->partition_edges, e1 = std::min<uint64_t>(g->m, e0 + g->partition_edges);
                 // (what is in a cache slot, or is copied into one now, needs no link)
-                h_direct[p] = h_hits[p] && !(hot && g->slot_of[p] >= 0) && h_hits[p] * 4 <= (e1 - e0) * 3 &&
-                              readable_in_place(g, e0, e1, need_w);
+                h_direct[p] = h_hits[p] && h_hits[p] * 4 <= (e1 - e0) * 3 && readable_in_place(g, e0, e1, need_w) &&
+                              !(hot && sparse_slot(g, p, e1 - e0, h_hits));
                 rr.parts_skipped += !h_hits[p];
                 active += h_hits[p];
                 if (h_direct[p]) {
@@ -924,7 +956,7 @@ void traverse_impl(ptg_graph *g, TravKind kind, uint32_t src, uint32_t *d_value,
                 uint64_t e0 = p * g->partition_edges;
                 uint64_t e1 = std::min<uint64_t>(g->m, e0 + g->partition_edges);
                 const uint32_t *sc_ = nullptr, *sw_ = nullptr;
-                const int slot = hot ? hot_slot(g, p, e1 - e0) : -1;
+                const int slot = hot ? hot_slot(g, p, e1 - e0, h_hits) : -1;
                 // a partition copies into a cache slot (kept for later levels and
                 // queries) or into the next staging buffer
                 bool copy_col = true, copy_w = need_w;

@@ -42,3 +42,30 @@ def test_streamed_traversals_match_oracle(ptg, ctx, oracle, name, wide, host, po
         assert (G.sssp(s, delta=delta) == dist).all()
     assert (G.cc() == oracle.cc(off, col)).all()
     G.close()
+
+
+@pytest.mark.parametrize("slots", [3, 64])
+@pytest.mark.parametrize("host", ["pinned", "pageable"])
+def test_sparse_rounds_fill_the_hot_cache(ptg, ctx, oracle, slots, host):
+    """PTG_RESIDENT_HOT where every round reads one vertex's edges: the partitions are promoted by
+    their visits all the same, so the next search needs less of the link (11 of 12 have a slot at most)."""
+    torch = pytest.importorskip("torch")
+    n, src, dst, s = chain(6000, 3)
+    off, col, w = csr(n, src, dst, True, n)
+    keep = None
+    if host == "pinned":
+        keep = [torch.from_numpy(a.view(np.int32)).pin_memory() for a in (col, w)]
+        col, w = [a.numpy().view(np.uint32) for a in keep]
+    cfg = ptg.partition_config(partition_bytes=8192, device_budget_bytes=(slots + 2) * 8192, force_out_of_core=1,
+                               hot_threshold=3600, resident_policy=ptg.PTG_RESIDENT_HOT)
+    G = ctx.graph(off, col, w, symmetric=False, config=cfg, pinned=host == "pinned")
+    assert G.info()["partitions"] == 12
+    dist = oracle.sssp(off, col, w, s)
+    first, second = {}, {}
+    assert (G.sssp(s, stats=first) == dist).all()
+    assert (G.sssp(s, stats=second) == dist).all()
+    assert second["partitions_cached"] > 0
+    assert second["link_bytes"] < first["link_bytes"]
+    if slots == 64:
+        assert second["link_bytes"] * 5 < first["link_bytes"]
+    G.close()
