@@ -241,13 +241,16 @@ typedef struct ptg_tuning {
     uint32_t expand_ctas_per_sm; /* CTAs per SM of the in-HBM traversals and the push
                                     relax of streamed graphs, 1..32 (default 4; the
                                     in-HBM kernel takes what fits, at most 4)            */
-    uint32_t pr_ctas_per_sm;     /* PageRank SpMV CTAs per SM, 1..32 (default 16)        */
+    uint32_t pr_ctas_per_sm;     /* PageRank SpMV CTAs per SM, 1..32 (default 16); at
+                                    most what an SM holds at once: 6, in passes of
+                                    several sources 5                                    */
     uint32_t pr_mid;             /* PageRank rows of 5..pr_mid edges run 8 lanes per
                                     row, longer ones a warp (default 256; 8..pr_chunk)   */
     uint32_t pr_chunk;           /* rows over pr_chunk edges are cut into pr_chunk-edge
-                                    pieces (default 4096; 128..65536); on graphs under
-                                    2^24 edges both are at most m / 4096 (256 or more)
-                                    and 1/16 of that (32 or more)                        */
+                                    pieces (default 4096; 128..65536).  Graphs under
+                                    2^24 edges: values up to the defaults are at most
+                                    m / 4096 (256 or more) and 1/16 of that (32 or
+                                    more), larger ones shrink in that proportion         */
     uint32_t ms_pull_small;      /* multi-source pull: rows up to this many edges take
                                     a thread, longer ones warps (default 32; 1..4096)    */
     uint32_t ms_pull_chunk;      /* edges per warp item of a long row (default 1024;

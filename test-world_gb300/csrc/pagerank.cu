@@ -683,6 +683,22 @@ __global__ void __launch_bounds__(kBlock) k_pr_bin_fill(const OffT *off, uint64_
     }
 }
 
+// Longest row of 8 lanes and edges per piece of a long row.  On a small graph
+// an iteration is as long as its longest unit of work, so rows are cut finer
+// there: pieces of m / 4096 edges (a power of two, 256 at least), 8 lanes a row
+// up to 1/16 of that (32 at least).  8 sources, 20 iterations, with 4096 / finer
+// pieces: 2^18 vertices 2.10 / 1.25 ms, 2^16 1.28 / 0.55, 2^14 0.99 / 0.25; one
+// source: 0.83 / 0.89, 0.44 / 0.41, 0.30 / 0.22.  Values tuned below the built-in ones
+// (256 and 4096) are limits besides; larger ones shrink in the same proportion.
+void pr_limits(const ptg_tuning &t, uint64_t m, uint32_t &mid, uint32_t &chunk) {
+    uint32_t fine = 256;
+    while (fine < 4096 && (uint64_t)fine * 2 * 4096 <= m) fine *= 2;
+    const uint32_t fine_mid = std::max(32u, fine / 16);
+    chunk = t.pr_chunk <= 4096 ? std::min(t.pr_chunk, fine) : (uint32_t)((uint64_t)t.pr_chunk * fine / 4096);
+    mid = t.pr_mid <= 256 ? std::min(t.pr_mid, fine_mid)
+                          : std::max(fine_mid, (uint32_t)((uint64_t)t.pr_mid * fine / 4096));
+}
+
 template <class OffT>
 void build_pr_bins(ptg_graph *g) {
     ptg_ctx *ctx = g->ctx;
@@ -691,15 +707,8 @@ void build_pr_bins(ptg_graph *g) {
     const int nb = (int)std::min<uint64_t>(1024, std::max<uint64_t>(1, (g->n + kBlock - 1) / kBlock));
     DevBuf counts;
     counts.ensure((uint64_t)nb * 4 * 8);
-    // On a small graph an iteration is as long as its longest unit of work, so
-    // rows are cut finer there: pieces of m / 4096 edges (a power of two, 256 at
-    // least), 8 lanes a row up to 1/16 of that.  8 sources, 20 iterations, with
-    // 4096 / finer pieces: 2^18 vertices 2.10 / 1.25 ms, 2^16 1.28 / 0.55, 2^14
-    // 0.99 / 0.25; one source: 0.83 / 0.89, 0.44 / 0.41, 0.30 / 0.22.
-    uint32_t fine = 256;
-    while (fine < 4096 && (uint64_t)fine * 2 * 4096 <= g->m) fine *= 2;
-    const uint32_t chunk = std::min(ctx->tuning.pr_chunk, fine);
-    const uint32_t mid = std::min(ctx->tuning.pr_mid, std::max(32u, chunk / 16));
+    uint32_t mid, chunk;
+    pr_limits(ctx->tuning, g->m, mid, chunk);
     launch(ctx, "k_pr_bin_count", k_pr_bin_count<OffT>, nb, kBlock, 0, st, off, g->n, mid, chunk,
            counts.as<unsigned long long>());
     std::vector<unsigned long long> h((size_t)nb * 4);
@@ -762,6 +771,9 @@ PrBins make_bins(ptg_graph *g, int sources, uint64_t warps, unsigned *&counters)
     return b;
 }
 
+// Warps take units until there are none, so CTAs past those that an SM holds at
+// once (ctas_per_sm) would only begin when the work is done: a tuning that asks
+// for more gets as many as fit.
 int pr_grid(ptg_graph *g, int ctas_per_sm, int sources, PrBins &bins) {
     const int per_sm = std::min(ctas_per_sm, (int)g->ctx->tuning.pr_ctas_per_sm);
     const uint64_t units = bins.n_items + bins.big_units + bins.mid_units + bins.small_units;
@@ -914,3 +926,8 @@ void run_pagerank(ptg_graph *g, bool personalized, uint32_t src, double damping,
 }
 
 }  // namespace ptg
+
+// For the tests: the limits that a graph of m edges gets.
+extern "C" void ptg_internal_pr_limits(const ptg_tuning *t, uint64_t m, uint32_t *mid, uint32_t *chunk) {
+    ptg::pr_limits(*t, m, *mid, *chunk);
+}

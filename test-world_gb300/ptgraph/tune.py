@@ -46,10 +46,10 @@ else:
 CANDIDATES = {
     "pr_mid": [16, 32, 64, 128, 256],
     "pr_chunk": [1024, 2048, 4096, 8192, 16384],
-    "pr_ctas_per_sm": [4, 6, 8, 12, 16],
+    "pr_ctas_per_sm": [2, 3, 4, 5, 16],  # (the built-in 16: as many as fit, 6)
     "bfs_alpha": [6.0, 10.0, 15.0, 22.0, 32.0],
     "bfs_beta": [8.0, 12.0, 18.0, 24.0, 36.0],
-    "expand_ctas_per_sm": [2, 3, 4, 6, 8, 12, 16],
+    "expand_ctas_per_sm": [1, 2, 3, 4],  # (4 of the in-HBM traversal fit)
     "sssp_delta_scale": [0.25, 0.5, 0.75, 1.0, 2.0, 4.0],
     "ms_pull_small": [8, 16, 32, 64, 128],
     "ms_pull_chunk": [256, 512, 1024, 2048, 4096],

@@ -272,3 +272,57 @@ def test_sweep_logic_without_gpu(ptg):
     assert doc["tuning"]["sssp_delta_scale"] == max(tune.CANDIDATES["sssp_delta_scale"])
     assert ctx.tuning() == doc["tuning"]
     json.dumps(doc)  # serialisable as written by the CLI
+
+
+def _pr_limits(ptg, m, **knobs):
+    import ctypes
+    t = ptg._tuning_struct(knobs)
+    mid, chunk = ctypes.c_uint32(), ctypes.c_uint32()
+    ptg.lib().ptg_internal_pr_limits(ctypes.byref(t), ctypes.c_uint64(m), ctypes.byref(mid), ctypes.byref(chunk))
+    return mid.value, chunk.value
+
+
+@pytest.mark.parametrize("m", [1, 1 << 20, (1 << 21) - 1, 1 << 22, 1 << 23, (1 << 24) - 1, 1 << 24, 1 << 33])
+def test_pagerank_bins_follow_the_tuning(ptg, m):
+    """From 2^24 edges on the tuned bins are the bins; below, larger values still make longer
+    pieces, and what is not tuned keeps the sizes that the graph calls for."""
+    fine = max(256, min(4096, 1 << max(0, (m // 4096).bit_length() - 1)))
+    assert _pr_limits(ptg, m) == (max(32, fine // 16), fine)
+    for chunk in (128, 1000, 4096, 8192, 16384, 65536):
+        for mid in (8, 16, 100, 256, 512, 8192, 65536):
+            if mid > chunk:
+                continue
+            got_mid, got_chunk = _pr_limits(ptg, m, pr_mid=mid, pr_chunk=chunk)
+            assert 8 <= got_mid <= got_chunk
+            if m >= 1 << 24:
+                assert (got_mid, got_chunk) == (mid, chunk)
+    assert len({_pr_limits(ptg, m, pr_chunk=c)[1] for c in (4096, 8192, 16384, 65536)}) == 4
+    assert len({_pr_limits(ptg, m, pr_mid=d, pr_chunk=65536)[0] for d in (256, 1024, 4096, 65536)}) >= (3 if m < 1 << 21 else 4)
+
+
+def test_sweep_values_are_different_runs(ptg):
+    """No two candidates of the autotuner make the same PageRank bins or launch (6 CTAs of the
+    PageRank pass and 4 of the traversal fit an SM)."""
+    from ptgraph import tune
+    m = 1 << 26  # the default sweep's graph has about so many
+    assert len({_pr_limits(ptg, m, pr_chunk=c) for c in tune.CANDIDATES["pr_chunk"]}) == len(tune.CANDIDATES["pr_chunk"])
+    assert len({_pr_limits(ptg, m, pr_mid=c) for c in tune.CANDIDATES["pr_mid"]}) == len(tune.CANDIDATES["pr_mid"])
+    for knob, fit in (("pr_ctas_per_sm", 6), ("expand_ctas_per_sm", 4)):
+        assert len({min(c, fit) for c in tune.CANDIDATES[knob]}) == len(tune.CANDIDATES[knob])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("knobs", [{"pr_chunk": 65536, "pr_mid": 8192}, {"pr_chunk": 16384}, {"pr_chunk": 1024, "pr_mid": 1024},
+                                   {"pr_chunk": 128, "pr_mid": 8}])
+def test_pagerank_with_tuned_bins(ptg, oracle, knobs):
+    """Bins well past and below the built-in ones, on a graph with rows of every bin."""
+    off, col, _ = ptg.gen_rmat(16, 16, seed=4, symmetric=True)
+    c = ptg.Ctx(0)
+    c.set_tuning(knobs)
+    G = c.graph(off, col, symmetric=True)
+    ref = oracle.pagerank(off, col)
+    assert (np.abs(G.pagerank().astype(np.float64) - ref) / ref).max() < PR_RTOL
+    rows = G.ppr_batch(np.array([0, 5, 77, 1000, 4000], np.uint32))
+    for i, s in enumerate([0, 5, 77, 1000, 4000]):
+        assert np.array_equal(rows[i].view(np.uint32), G.ppr(s).view(np.uint32))
+    c.close()
