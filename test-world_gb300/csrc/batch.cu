@@ -17,6 +17,7 @@ namespace ptg {
 bool ms_group(ptg_graph *g, const uint32_t *h_srcs, uint32_t k, uint32_t *d_rows, bool weighted,
               uint32_t flags, RunResult &rr);
 uint32_t ms_group_size(bool weighted);
+void ms_done(ptg_ctx *ctx);
 }
 
 extern "C" {
@@ -59,6 +60,7 @@ static ptg_status ms_common(ptg_graph *g, const uint32_t *sources, uint32_t k, u
         }
         PTG_CUDA_TRY(cudaEventRecord(ctx->ev1, st));
         PTG_CUDA_TRY(cudaStreamSynchronize(st));
+        ms_done(ctx);
         ctx->prof.resolve();
         float ms = 0;
         cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);

@@ -181,6 +181,34 @@ struct MsHist {
     const u64 *m[kMsHist];
 };
 
+// Room for the frontier masks of consecutive levels in ws.ms[0]; returns how many.
+// Fewer than kMsHist only cost further passes over the rows, so the masks past
+// the two that a level needs take at most a quarter of the free memory (or the
+// room that a server gives its lane); up to a 64th of the device's memory they
+// are taken without asking.
+int ms_history(ptg_ctx *ctx, uint64_t mask_bytes) {
+    DevBuf &b = ctx->ws.ms[0];
+    uint64_t room = ctx->mask_room;
+    if (room == ~0ull && b.bytes < kMsHist * mask_bytes && kMsHist * mask_bytes > ctx->hbm_bytes / 64) {
+        size_t dfree = 0, total = 0;
+        PTG_CUDA_TRY(device_free_bytes(ctx->device, &dfree, &total));
+        room = (dfree + b.bytes) / 4;
+    } else if (room != ~0ull && b.bytes > 2 * mask_bytes + room + room / 8 + (8ull << 20)) {
+        b.release();  // a server whose budget has shrunk
+    }
+    int hist = (int)std::min<uint64_t>(kMsHist, 2 + room / mask_bytes);
+    while (true) {
+        try {
+            b.ensure(hist * mask_bytes);
+            return hist;
+        } catch (const Error &e) {
+            if (e.status != PTG_ERR_OOM || hist == 2) throw;
+            cudaGetLastError();
+            hist = std::max(2, hist / 2);
+        }
+    }
+}
+
 // Rows out of the kept levels: out[s*n + v] = level0 + l for the level l whose
 // mask holds source s at v (at newid[v] on a regrouped graph).  FIRST: every
 // word is written, unreached where no level has it; else only the found ones.
@@ -905,19 +933,11 @@ void msbfs_impl(ptg_graph *g, const uint32_t *h_srcs, uint32_t k, uint32_t *d_ro
     const uint32_t *col = g->d_col.as<uint32_t>();
     uint32_t base = (flags & PTG_LEVEL_ZERO_BASED) ? 0u : 1u;
     ms_prepare<OffT>(g);
-    // ms[0]: the levels' frontier masks, as many as there is memory for (two
-    // at least: a level and the next); ms[1]: sources seen per vertex
+    // ms[0]: the levels' frontier masks (two at least: a level and the next);
+    // ms[1]: sources seen per vertex
     const uint64_t mask_words = (n * W + 31) / 32 * 32, mask_bytes = mask_words * 8;
     ws.ms[1].ensure(mask_bytes);
-    int hist = kMsHist;
-    try {
-        ws.ms[0].ensure(hist * mask_bytes);
-    } catch (const Error &e) {
-        if (e.status != PTG_ERR_OOM) throw;
-        cudaGetLastError();
-        hist = 2;
-        ws.ms[0].ensure(hist * mask_bytes);
-    }
+    const int hist = ms_history(ctx, mask_bytes);
     if (g->symmetric && !g->pull_items_built) build_pull_items<OffT>(g);
     u64 *S = ws.ms[1].as<u64>();
     MsHist h{};
@@ -1111,6 +1131,13 @@ void ms_prepare_graph(ptg_graph *g) {
 // Sources per fused group: 256 for BFS (4 mask words), 64 for SSSP.
 uint32_t ms_group_size(bool weighted) { return weighted ? 64u : 256u; }
 
+// The masks go back to the device's block cache after a call (from where the next
+// one takes them) unless they are small: they are up to 13 x 32 bytes per vertex,
+// memory that a graph created meanwhile may need.
+void ms_done(ptg_ctx *ctx) {
+    if (ctx->ws.ms[0].bytes > (256ull << 20)) ctx->ws.ms[0].release();
+}
+
 // One group of at most ms_group_size() sources; d_rows receives k rows of n
 // values.  Returns false when the fused path does not apply (out-of-core).
 bool ms_group(ptg_graph *g, const uint32_t *h_srcs, uint32_t k, uint32_t *d_rows, bool weighted,
@@ -1122,7 +1149,7 @@ bool ms_group(ptg_graph *g, const uint32_t *h_srcs, uint32_t k, uint32_t *d_rows
         else mssssp_impl<uint32_t>(g, h_srcs, k, d_rows, flags, rr);
     } else {
         // levels go to the rows once, by caller id, from the kept masks
-                if (k <= 64) {
+        if (k <= 64) {
             if (o64) msbfs_impl<unsigned long long, 1>(g, h_srcs, k, d_rows, flags, rr);
             else msbfs_impl<uint32_t, 1>(g, h_srcs, k, d_rows, flags, rr);
         } else if (k <= 128) {

@@ -269,6 +269,9 @@ struct ptg_ctx {
     ptg::Prof prof;
     ptg::Workspace ws;
     ptg_tuning tuning;                   // ptg_tuning_defaults at creation
+    // bytes that a multi-source BFS may keep levels' masks in, past the two it
+    // needs (set by a server for its lane; ~0: by the free memory)
+    uint64_t mask_room = ~0ull;
 };
 
 namespace ptg {

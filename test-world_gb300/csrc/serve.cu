@@ -91,7 +91,7 @@ uint64_t batch_bytes(uint32_t kind, uint64_t n, uint64_t m, uint32_t k, bool reg
     if (regrouped) q += 2 * n * 4;
     if (kind == PTG_Q_BFS) {
         uint64_t W = k <= 64 ? 1 : (k <= 128 ? 2 : 4);
-        return 13 * n * 8 * W + rows + q;  // 12 levels' masks and the seen mask
+        return 3 * n * 8 * W + rows + q;  // two levels' masks and the seen mask; more where there is room
     }
     if (kind == PTG_Q_SSSP) return n * 66 * 4 + 2 * n * 8 + rows + q;
     return 2 * n * 32 * 4 + rows + (m / 2048 + 1) * 32 * 8;  // PPR
@@ -208,9 +208,9 @@ struct Batch {
     std::vector<uint64_t> ids;
     std::vector<uint32_t> srcs;
     std::vector<void *> results;
+    uint64_t spare = 0;  // what the batch leaves of the lane's share of the memory budget
 };
 
-// Under s->mu: take the next batch for lane li, or return false.
 // Estimated device time per request (ms) of serving k requests of a group the
 // cheaper way (fused pass or single queries); negative while unmeasured.
 double per_request_ms(const Entry &e, uint32_t kd, uint32_t k) {
@@ -221,6 +221,17 @@ double per_request_ms(const Entry &e, uint32_t kd, uint32_t k) {
     return f > 0 && f < k * single ? f / k : single;
 }
 
+// A lane's share of what the memory budget leaves (under s->mu).
+uint64_t lane_share(const ptg_server *s) {
+    return (s->budget > s->graph_bytes ? s->budget - s->graph_bytes : 0) / s->lanes.size();
+}
+
+uint64_t spare_bytes(const ptg_server *s, const ptg_graph *g, uint32_t kind, uint32_t k) {
+    const uint64_t share = lane_share(s), need = batch_bytes(kind, g->n, g->m, k, g->relabeled);
+    return share > need ? share - need : 0;
+}
+
+// Under s->mu: take the next batch, or return false.
 bool take_batch(ptg_server *s, Batch &b) {
     if (s->inflight >= s->cfg.max_slots) return false;
     // Which group: the one holding the oldest request (PTG_SCHEDULE_OLDEST;
@@ -260,8 +271,7 @@ bool take_batch(ptg_server *s, Batch &b) {
     uint32_t k = e.g->out_of_core ? 1u : kind_max(s, best->first.second);
     k = (uint32_t)std::min<uint64_t>(k, s->cfg.max_slots - s->inflight);
     k = (uint32_t)std::min<uint64_t>(k, best->second.size());
-    uint64_t left = s->budget > s->graph_bytes ? s->budget - s->graph_bytes : 0;
-    uint64_t share = left / s->lanes.size();
+    const uint64_t share = lane_share(s);
     const uint32_t kd = best->first.second;
     while (k > 1 && batch_bytes(kd, n, m, k, e.g->relabeled) > share) k = (k + 1) / 2;
     // one fused pass for k requests, or a single-source query: whichever the
@@ -274,6 +284,7 @@ bool take_batch(ptg_server *s, Batch &b) {
     else b.fused = (k <= small_k(kd) && e.fused_small_ms[kd] > 0 ? e.fused_small_ms[kd] : e.fused_ms[kd]) <
                    k * e.single_ms[kd];
     if (!b.fused) k = 1;
+    b.spare = spare_bytes(s, e.g, kd, k);
     b.ent = &e;
     b.graph = best->first.first;
     b.kind = kd;
@@ -313,6 +324,7 @@ ptg_status run_batch(ptg_server *s, Lane &L, size_t li, const Batch &b) {
     return guard(ctx, [&] {
         PTG_CUDA_TRY(cudaSetDevice(ctx->device));
         const uint64_t n = v->n;
+        ctx->mask_room = b.spare;
         L.rows.ensure((uint64_t)k * n * 4);
         RunResult rr;
         const double d = s->cfg.ppr_damping > 0 ? s->cfg.ppr_damping : 0.85;
@@ -426,6 +438,10 @@ void calibrate(ptg_server *s, uint32_t gid) {
             b.ids.push_back(0);
             b.srcs.push_back(src[i % src.size()]);
             b.results.push_back(scratch.p);
+        }
+        {
+            std::lock_guard<std::mutex> lk(s->mu);
+            b.spare = spare_bytes(s, g, kind, k);
         }
         if (run_batch(s, *s->lanes[0], 0, b) != PTG_OK) return -1;  // warm-up: workspace growth
         auto t0 = Clock::now();

@@ -70,3 +70,45 @@ def test_dense_sssp_rounds(ptg, ctx, ctx_grouped, oracle, grouped, both_ways, n,
     for i, s in enumerate(srcs):
         assert (dist[i] == oracle.sssp(off, col.astype(np.uint32), w, int(s))).all()
     G.close()
+
+
+def test_level_masks_are_given_back(ptg):
+    """What a call of 256 sources kept its levels in (12 x 32 MB here) is free for others after it."""
+    torch = pytest.importorskip("torch")
+    n, k = 1 << 20, 256
+    rng = np.random.RandomState(1)
+    key = np.unique(rng.randint(0, n, 1 << 22).astype(np.int64) * n + rng.randint(0, n, 1 << 22))
+    off = np.zeros(n + 1, np.uint64)
+    off[1:] = np.cumsum(np.bincount(key // n, minlength=n))
+    c = ptg.Ctx(0)
+    G = c.graph(off, (key % n).astype(np.uint32))
+    out = torch.empty((k, n), dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    before = c.device_info()["free_bytes"]
+    G.msbfs(rng.randint(0, n, k).astype(np.uint32), flags=ptg.PTG_OUT_DEVICE, out=out)
+    kept = before - c.device_info()["free_bytes"]
+    assert kept < 3 * 32 * n + (64 << 20)  # a level, the next and the seen mask, queues and scans
+    c.close()
+
+
+@pytest.mark.parametrize("masks", [0, 1, 3, 5, 30])
+def test_served_batches_fit_the_budget(ptg, oracle, masks):
+    """A lane's batches are sized by the three masks that a level needs, and keep as many levels
+    as the budget has room for besides."""
+    n, k = 1 << 14, 256
+    off, col, _ = chain_with_leaves(40, n, 3)
+    m = col.size
+    need = 3 * 32 * n + 4 * k * n + 8 * n + 16 * (n + 1) + 4 * (m // 2048 + 4)
+    c = ptg.Ctx(0)
+    G = c.graph(off, col, symmetric=True)
+    assert not G.info()["degree_grouped"]
+    srv = ptg.Server(c, lanes=1, max_slots=2 * k, memory_budget_bytes=need + masks * 32 * n + 64)
+    gid = srv.add_graph(G)
+    srcs = [int(s) for s in np.random.RandomState(masks).randint(0, n, 600)]
+    ids = [srv.submit(gid, ptg.PTG_Q_BFS, s) for s in srcs]
+    rows = [srv.wait(i)[0] for i in ids]
+    st = srv.stats()
+    assert st["max_batch_seen"] == k
+    for s, row in list(zip(srcs, rows))[::20]:
+        assert (row == oracle.bfs(off, col, s, method="queue")).all()
+    c.close()
