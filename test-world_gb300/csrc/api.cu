@@ -1080,4 +1080,10 @@ void ptg_compat_set_partition_config(const ptg_partition_config *cfg) {
 }
 void ptg_compat_set_device(int device) { tls.device = device; }
 
+// For the tests: how long a traversal's blocks wait at their barrier.
+void ptg_internal_set_barrier_polls(ptg_ctx *ctx, uint64_t polls) {
+    std::lock_guard<std::mutex> lk(ctx->mu);
+    ctx->barrier_polls = polls;
+}
+
 }  // extern "C"

@@ -272,6 +272,8 @@ struct ptg_ctx {
     // bytes that a multi-source BFS may keep levels' masks in, past the two it
     // needs (set by a server for its lane; ~0: by the free memory)
     uint64_t mask_room = ~0ull;
+    // polls of a traversal's grid barrier before a block gives up (tens of seconds)
+    uint64_t barrier_polls = 1ull << 26;
 };
 
 namespace ptg {

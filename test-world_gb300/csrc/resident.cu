@@ -75,8 +75,6 @@ constexpr unsigned kErrOverflow = 1u, kErrBarrier = 2u, kErrLimit = 4u;
 // relaxations.  RMAT-24 from width 6: 24 rounds and 4.2 ms a search, 45 rounds
 // and 4.5 ms without.
 constexpr u64 kWideEdges = 1ull << 21;
-// polls of the barrier before a CTA gives up (tens of seconds)
-constexpr u64 kBarrierPolls = 1ull << 26;
 
 // Every thread takes the launch's decisions for itself, from words that it reads
 // after a barrier.  A thread may be late with that read (another lane's kernels on
@@ -132,6 +130,7 @@ struct ResArgs {
     ResCtl *ctl;
     LevelMsg *msg;                  // where the outcome goes (host-mapped, or ctl->msg)
     uint32_t seq;
+    u64 barrier_polls;              // polls of the barrier before a CTA gives up
 };
 
 
@@ -141,8 +140,10 @@ __device__ __forceinline__ unsigned ld_acquire(const unsigned *p) {
     return v;
 }
 
-// All CTAs of the (cooperative) grid meet; false when one of them gave up.
-__device__ bool grid_barrier(ResCtl *c) {
+// All CTAs of the (cooperative) grid meet; false when one of them gave up.  Who
+// passes knows that all others had reached it, so what was written before it is
+// complete even when a CTA gives up at it.
+__device__ bool grid_barrier(ResCtl *c, u64 limit) {
     __shared__ int s_ok;
     __syncthreads();
     if (gridDim.x == 1) {
@@ -162,7 +163,7 @@ __device__ bool grid_barrier(ResCtl *c) {
             u64 polls = 0;
             while (ld_acquire(&c->gen) == gen) {
                 if ((++polls & 1023u) == 0 && (*(volatile unsigned *)&c->error & kErrBarrier)) ok = false;
-                if (polls > kBarrierPolls) {
+                if (polls > limit) {
                     atomicOr(&c->error, kErrBarrier);
                     ok = false;
                 }
@@ -728,7 +729,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_traverse(ResArgs a) {
         for (int i = 0; i < 2; i++) ctl->pull_edges[i] = ctl->pull_items[i] = ctl->pull_bigs[i] = 0;
         ctl->error = 0;
     }
-    if (!grid_barrier(ctl)) return;
+    if (!grid_barrier(ctl, a.barrier_polls)) return;
     bool queued = MODE != 2;  // the current frontier is in the queue (else only in its bitmap, or all vertices)
     if (MODE != 2) {
         if (blockIdx.x == 0) {
@@ -752,7 +753,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_traverse(ResArgs a) {
                 ctl->edges[0] = deg;
             }
         }
-        if (!grid_barrier(ctl)) return;
+        if (!grid_barrier(ctl, a.barrier_polls)) return;
     }
 
     uint64_t m_unvisited = a.m, edges_done = 0;
@@ -826,7 +827,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_traverse(ResArgs a) {
             buf_finish<OffT>(buf, a, front, &ctl->bucket_found[far_turn % 3], &ctl->bucket_edges[far_turn % 3]);
             thr = to;
             far_turn++;
-            if (!grid_barrier(ctl)) return;
+            if (!grid_barrier(ctl, a.barrier_polls)) return;
             continue;
         }
         scanned = false;
@@ -884,7 +885,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_traverse(ResArgs a) {
                 }
                 sum = block_reduce_sum(sum);
                 if (threadIdx.x == 0 && sum) atomicAdd(&ctl->pull_edges[turn], sum);
-                if (!grid_barrier(ctl)) return;
+                if (!grid_barrier(ctl, a.barrier_polls)) return;
                 pull_E = ctl->pull_edges[turn];
                 sssp_pull = pull_E < most;
                 if (leader) ctl->pull_edges[turn ^ 1] = ctl->pull_items[turn ^ 1] = ctl->pull_bigs[turn ^ 1] = 0;
@@ -901,7 +902,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_traverse(ResArgs a) {
             const Frontier nx = frontier_of(a, cur ^ 1, next);
             WarpBuf longer{s_look[wid], 0, PTG_UNREACHED, 0, 0};
             sssp_pull_few<OffT>(a, above, thr, bm_next, nx, buf, look, longer);
-            if (!grid_barrier(ctl)) return;
+            if (!grid_barrier(ctl, a.barrier_polls)) return;
             sssp_pull_longer<OffT>(a, look, thr, bm_next, nx, buf, &ctl->found[next], &ctl->edges[next]);
         } else if (MODE == 0 && bottom_up) {
             // few unvisited vertices left: what the last pull round looked at and did not find
@@ -916,7 +917,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_traverse(ResArgs a) {
                 // its queue, and a clear bitmap for the next one
                 queue_bits<OffT>(a, MODE == 2 ? nullptr : bm_cur, front, buf);
                 for (uint64_t i = tid; i < words; i += nthreads) bm_next[i] = 0u;
-                if (!grid_barrier(ctl)) return;
+                if (!grid_barrier(ctl, a.barrier_polls)) return;
                 queued = true;
             }
             edges_done += E;
@@ -927,13 +928,13 @@ __global__ void __launch_bounds__(kBlock, 4) k_traverse(ResArgs a) {
                                    frontier_of(a, cur ^ 1, next), buf,
                                    &ctl->found[next], &ctl->edges[next]);
         }
-        if (!grid_barrier(ctl)) return;
+        if (!grid_barrier(ctl, a.barrier_polls)) return;
         cur ^= 1;
         level++;
     }
     if (MODE == 1 && a.out) {  // the values by caller id
         for (uint64_t v = tid; v < a.n; v += nthreads) a.out[v] = a.value[a.newid[v]];
-        if (!grid_barrier(ctl)) return;
+        if (!grid_barrier(ctl, a.barrier_polls)) return;
     }
     if (leader) {  // everything was written before the last barrier
         volatile LevelMsg *m = a.msg;
@@ -1049,6 +1050,7 @@ void run_resident(ptg_graph *g, TravKind kind, uint32_t src, uint32_t *d_value, 
     a.base = base;
     a.delta = delta;
     a.max_iters = max_iters;
+    a.barrier_polls = ctx->barrier_polls;
     a.alpha = ctx->tuning.bfs_alpha;
     a.beta = ctx->tuning.bfs_beta;
     a.use_far = kind == TRAV_SSSP && delta != 0;
@@ -1089,7 +1091,12 @@ void run_resident(ptg_graph *g, TravKind kind, uint32_t src, uint32_t *d_value, 
         }
         PTG_REQUIRE(done.seq == a.seq, PTG_ERR_TIMEOUT, "a traversal's blocks did not all reach a barrier");
     } catch (const Error &) {
+        // did the launch end at a barrier?  (Its CTAs publish nothing then.)
+        unsigned error = 0;
+        const bool gave_up = cudaMemcpyAsync(&error, &a.ctl->error, sizeof(error), cudaMemcpyDeviceToHost, st) == cudaSuccess &&
+                             cudaStreamSynchronize(st) == cudaSuccess && (error & kErrBarrier);
         ws.res.release();  // a barrier that was left half-way is not used again
+        PTG_REQUIRE(!gave_up, PTG_ERR_TIMEOUT, "a traversal's blocks did not all reach a barrier");
         throw;
     }
     PTG_REQUIRE(!(done.error & kErrOverflow), PTG_ERR_CUDA, "frontier overflow in relax");

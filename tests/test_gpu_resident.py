@@ -188,3 +188,27 @@ def test_bucket_width_past_every_distance(ptg, ctx, oracle, name, delta, zero_ba
     want = np.where(dist == 0xFFFFFFFF, dist, dist - 1) if zero_based else dist
     assert (G.sssp(s, delta=delta, flags=ptg.PTG_LEVEL_ZERO_BASED if zero_based else 0) == want).all()
     G.close()
+
+
+@pytest.mark.parametrize("kind", ["bfs", "sssp", "cc"])
+def test_barrier_wait_runs_out(ptg, oracle, kind):
+    """Blocks that wait for the others at most one poll give up: the call reports a timeout, and the
+    context answers the next call."""
+    import ctypes
+    n, src, dst, s = GRAPHS["large"]()
+    off, col, w = csr(n, src, dst, True, n)
+    c = ptg.Ctx(0)
+    G = c.graph(off, col, w, symmetric=True)
+    call = {"bfs": lambda: G.bfs(s), "sssp": lambda: G.sssp(s), "cc": lambda: G.cc(flags=ptg.PTG_REFERENCE_SCHEDULE)}[kind]
+    want = {"bfs": lambda: oracle.bfs(off, col, s, method="queue"), "sssp": lambda: oracle.sssp(off, col, w, s),
+            "cc": lambda: oracle.cc(off, col)}[kind]()
+    polls = ptg.lib().ptg_internal_set_barrier_polls
+    for _ in range(3):
+        polls(c.h, ctypes.c_uint64(1))
+        with pytest.raises(ptg.PtgError) as e:
+            call()
+        assert e.value.status == ptg.PTG_ERR_TIMEOUT
+        assert "barrier" in str(e.value)
+        polls(c.h, ctypes.c_uint64(1 << 26))
+        assert (call() == want).all()
+    c.close()
