@@ -269,12 +269,15 @@ void ensure_level_msg(Workspace &ws) {
 // The outcome of the level (or multi-source round) just queued (message
 // ws.msg_seq), read from mapped host memory once its last kernel has
 // published it.  While waiting, the stream is asked now and then
-// whether it has failed, or finished without the message; a level that
-// takes longer than ten minutes is reported as a timeout.
-LevelMsg wait_level_msg(Workspace &ws, cudaStream_t st) {
+// whether it has failed, or finished without the message; ten minutes
+// without it are reported as a timeout, counted anew whenever a traversal,
+// which is one launch for all of its levels, has said that it goes on.
+LevelMsg wait_level_msg(ptg_ctx *ctx, cudaStream_t st) {
+    Workspace &ws = ctx->ws;
     LevelMsg *m = ws.h_msg.as<LevelMsg>();
     const uint32_t want = ws.msg_seq;
-    const auto t0 = std::chrono::steady_clock::now();
+    auto t0 = std::chrono::steady_clock::now();
+    auto steps = __atomic_load_n(&m->frontier_E, __ATOMIC_RELAXED);
     for (uint64_t it = 1; __atomic_load_n(&m->seq, __ATOMIC_ACQUIRE) != want; it++) {
         if (it % 1024 != 0) continue;
         const cudaError_t e = cudaStreamQuery(st);
@@ -283,7 +286,13 @@ LevelMsg wait_level_msg(Workspace &ws, cudaStream_t st) {
             throw Error{PTG_ERR_CUDA, "traversal level finished without publishing its outcome"};
         }
         if (e != cudaErrorNotReady) PTG_CUDA_TRY(e);
-        if (std::chrono::steady_clock::now() - t0 > std::chrono::minutes(10))
+        const auto now = std::chrono::steady_clock::now();
+        const auto got = __atomic_load_n(&m->frontier_E, __ATOMIC_RELAXED);
+        if (got != steps) {
+            steps = got;
+            t0 = now;
+        }
+        if (now - t0 > std::chrono::milliseconds(ctx->wait_ms))
             throw Error{PTG_ERR_TIMEOUT, "traversal level did not finish within ten minutes"};
     }
     LevelMsg out;
@@ -1080,10 +1089,15 @@ void ptg_compat_set_partition_config(const ptg_partition_config *cfg) {
 }
 void ptg_compat_set_device(int device) { tls.device = device; }
 
-// For the tests: how long a traversal's blocks wait at their barrier.
+// For the tests: how long a traversal's blocks wait at their barrier, and the host
+// for a level message.
 void ptg_internal_set_barrier_polls(ptg_ctx *ctx, uint64_t polls) {
     std::lock_guard<std::mutex> lk(ctx->mu);
     ctx->barrier_polls = polls;
+}
+void ptg_internal_set_wait_ms(ptg_ctx *ctx, uint32_t ms) {
+    std::lock_guard<std::mutex> lk(ctx->mu);
+    ctx->wait_ms = ms;
 }
 
 }  // extern "C"

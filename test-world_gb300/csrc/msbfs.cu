@@ -901,7 +901,7 @@ inline void ms_next(ptg_ctx *ctx, Workspace &ws, uint64_t &F, uint64_t &Eact, ui
     if (ws.d_msg) {
         launch(ctx, "k_ms_round_end", k_ms_round_end, 1, 1, 0, st, d_ctl, ws.d_msg, ws.msg_seq + 1);
         ws.msg_seq++;
-        const LevelMsg msg = wait_level_msg(ws, st);
+        const LevelMsg msg = wait_level_msg(ctx, st);
         PTG_REQUIRE(msg.error == 0, PTG_ERR_CUDA, "frontier overflow in multi-source round");
         F = msg.F;
         Eact = msg.frontier_E;

@@ -234,7 +234,7 @@ struct LevelMsg {
     uint32_t F;      // rounds: the next frontier's size; traversals: levels run
     uint32_t error;  // error bits
     uint32_t pad;    // traversals: pull levels
-    unsigned long long frontier_E;  // rounds: edges of the next frontier
+    unsigned long long frontier_E;  // rounds: edges of the next frontier; traversals: steps so far
     unsigned long long E;           // edges scanned
 };
 
@@ -250,7 +250,7 @@ struct Workspace {
 };
 
 void ensure_level_msg(Workspace &ws);
-LevelMsg wait_level_msg(Workspace &ws, cudaStream_t st);
+LevelMsg wait_level_msg(ptg_ctx *ctx, cudaStream_t st);
 
 struct Graph;
 
@@ -274,6 +274,8 @@ struct ptg_ctx {
     uint64_t mask_room = ~0ull;
     // polls of a traversal's grid barrier before a block gives up (tens of seconds)
     uint64_t barrier_polls = 1ull << 26;
+    // how long the host waits for a level message without a sign of progress
+    uint32_t wait_ms = 600000;
 };
 
 namespace ptg {

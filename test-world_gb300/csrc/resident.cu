@@ -759,12 +759,16 @@ __global__ void __launch_bounds__(kBlock, 4) k_traverse(ResArgs a) {
     uint64_t m_unvisited = a.m, edges_done = 0;
     u64 front_E = 0;
     uint32_t iterations = 0, pulls = 0, level = 0, far_turn = 0, pull_turn = 0, late_pulls = 0;
-    uint32_t thr = PTG_UNREACHED;
+    uint32_t thr = PTG_UNREACHED, steps = 0;
     u64 delta = a.delta, bucket_E = 0;
     if (MODE == 1 && a.use_far) thr = bucket_end(a.base, a.delta);
     bool bottom_up = false, limit = false, scanned = false;
     int cur = 0;
     while (true) {
+        // a sign of life for the host, which bounds its wait (a path of 10^8
+        // vertices has as many levels); seldom, as a store to host memory holds up
+        // the next fence
+        if (leader && (++steps & 63u) == 0) ((volatile LevelMsg *)a.msg)->frontier_E = steps;
         const int slot = level % 3, next = (level + 1) % 3, later = (level + 2) % 3;
         // (after a bucket pass: what it took, the round before had found nothing)
         u64 F = scanned ? ctl->bucket_found[(far_turn + 2) % 3] : ctl->found[slot];
@@ -1084,7 +1088,7 @@ void run_resident(ptg_graph *g, TravKind kind, uint32_t src, uint32_t *d_value, 
         if (g->off64) resident_impl<unsigned long long>(g, kind, a);
         else resident_impl<uint32_t>(g, kind, a);
         if (ws.d_msg) {
-            done = wait_level_msg(ws, st);
+            done = wait_level_msg(ctx, st);
         } else {
             PTG_CUDA_TRY(cudaMemcpyAsync(&done, a.msg, sizeof(done), cudaMemcpyDeviceToHost, st));
             PTG_CUDA_TRY(cudaStreamSynchronize(st));

@@ -212,3 +212,27 @@ def test_barrier_wait_runs_out(ptg, oracle, kind):
         polls(c.h, ctypes.c_uint64(1 << 26))
         assert (call() == want).all()
     c.close()
+
+
+def test_long_searches_are_waited_for(ptg, oracle):
+    """A search is one launch: the host's limit counts from its last sign of life, not from its start.
+    (100 K levels, some 0.6 s, with a limit of 50 ms.)  Without any sign the call reports a timeout,
+    and the context answers the next one."""
+    import ctypes
+    n, src, dst, s = chain(100000, 5)
+    off, col, w = csr(n, src, dst, True, 0)
+    c = ptg.Ctx(0)
+    G = c.graph(off, col, w, symmetric=True)
+    want = oracle.bfs(off, col, s, method="queue")
+    wait = ptg.lib().ptg_internal_set_wait_ms
+    assert (G.bfs(s) == want).all()
+    wait(c.h, ctypes.c_uint32(50))
+    assert (G.bfs(s) == want).all()
+    assert (G.sssp(s, delta=1) == oracle.sssp(off, col, w, s)).all()
+    wait(c.h, ctypes.c_uint32(0))
+    with pytest.raises(ptg.PtgError) as e:
+        G.bfs(s)
+    assert e.value.status == ptg.PTG_ERR_TIMEOUT
+    wait(c.h, ctypes.c_uint32(600000))
+    assert (G.bfs(s) == want).all()
+    c.close()
