@@ -43,6 +43,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <random>
 
 #include "frontier.cuh"
 
@@ -505,16 +506,18 @@ __global__ void __launch_bounds__(kBlock) k_relax_partition(uint64_t e_begin, ui
 // Whether every edge carries the same weight both ways: sum over the edges
 // u < v of a hash of (u, v, w), less the same over the edges u > v; zero when the
 // two lists of (smaller end, larger end, weight) are the same (and, where they
-// differ, with probability 2^-64).  Also the weights' sum and minimum, as
-// k_weight_sum.  A warp walks an equal run of edges, 8 consecutive ones per
-// lane and step; the rows that begin in a step's 256 edges are written at their
-// first edge in shared memory, and a running maximum gives each edge its row.
-// (Tiles of a CTA with a search of their row bounds each: 3.07 ms on RMAT-24,
-// 1.83 now; half of it is the hash.)
+// differ, with a probability of about 2^-64: the hash is keyed with a random
+// number per check, as weights can be chosen that defeat a fixed one).  Also the
+// weights' sum and minimum, as k_weight_sum.  A warp walks an equal run of edges,
+// 8 consecutive ones per lane and step; the rows that begin in a step's 256 edges
+// are written at their first edge in shared memory, and a running maximum gives
+// each edge its row.  (Tiles of a CTA with a search of their row bounds each: 3.07
+// ms on RMAT-24, 1.83 now; half of it is the hash.)
 constexpr uint32_t kBalStep = 256;
 template <class OffT>
 __global__ void __launch_bounds__(kBlock, 4) k_weight_balance(uint64_t m, uint64_t n, const OffT *off, const uint32_t *col,
-                                                              const uint32_t *w, unsigned long long *out) {
+                                                              const uint32_t *w, unsigned long long key,
+                                                              unsigned long long *out) {
     constexpr int kEach = kBalStep / 32;
     __shared__ __align__(16) uint32_t s_row[kBlock / 32][kBalStep];
     uint32_t *rows = s_row[threadIdx.x >> 5];
@@ -578,7 +581,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_weight_balance(uint64_t m, uint64
             least = min(least, ws[i]);
             if (j0 + i >= t1) continue;
             const uint32_t u = max(at[i], before), v = vs[i];
-            unsigned long long h = ((unsigned long long)min(u, v) << 32 | max(u, v)) * 0x9E3779B97F4A7C15ull;
+            unsigned long long h = (((unsigned long long)min(u, v) << 32 | max(u, v)) ^ key) * 0x9E3779B97F4A7C15ull;
             h = (h ^ (h >> 32) ^ ws[i]) * 0xBF58476D1CE4E5B9ull;
             h = (h ^ (h >> 32)) * 0x94D049BB133111EBull;
             h ^= h >> 32;
@@ -1073,12 +1076,14 @@ bool graph_weights_symmetric(ptg_graph *g) {
             unsigned long long h[3] = {0, 0, 0xFFFFFFFFull};
             PTG_CUDA_TRY(cudaMemcpyAsync(acc, h, 24, cudaMemcpyHostToDevice, st));
             const int grid = grid_for(g->m, kTile, ctx->sm_count * 4);
+            std::random_device rd;
+            const unsigned long long key = (unsigned long long)rd() << 32 | rd();
             if (g->off64)
                 launch(ctx, "k_weight_balance", k_weight_balance<unsigned long long>, grid, kBlock, 0, st, g->m, g->n,
-                       g->d_off.as<unsigned long long>(), g->d_col.as<uint32_t>(), g->d_w.as<uint32_t>(), acc);
+                       g->d_off.as<unsigned long long>(), g->d_col.as<uint32_t>(), g->d_w.as<uint32_t>(), key, acc);
             else
                 launch(ctx, "k_weight_balance", k_weight_balance<uint32_t>, grid, kBlock, 0, st, g->m, g->n,
-                       g->d_off.as<uint32_t>(), g->d_col.as<uint32_t>(), g->d_w.as<uint32_t>(), acc);
+                       g->d_off.as<uint32_t>(), g->d_col.as<uint32_t>(), g->d_w.as<uint32_t>(), key, acc);
             PTG_CUDA_TRY(cudaMemcpyAsync(h, acc, 24, cudaMemcpyDeviceToHost, st));
             PTG_CUDA_TRY(cudaStreamSynchronize(st));
             set_weight_stats(g, h[1], (uint32_t)h[2]);

@@ -112,3 +112,19 @@ def test_served_batches_fit_the_budget(ptg, oracle, masks):
     for s, row in list(zip(srcs, rows))[::20]:
         assert (row == oracle.bfs(off, col, s, method="queue")).all()
     c.close()
+
+
+@pytest.mark.parametrize("out_weights,back_weights", [
+    ((158294597, 252129289, 84674016, 232866233), (169702344, 154819396, 62669269, 58675956)),
+    ((251776810, 242173211, 73729864, 188310061), (19052126, 157150182, 155272291, 72500844)),
+])
+def test_weights_chosen_to_look_symmetric(ptg, ctx, oracle, out_weights, back_weights):
+    """A star whose edges weigh something else outwards than back, with weights for which the sums
+    of an unkeyed hash agree: its rounds must not take the one for the other."""
+    off = np.array([0, 4, 5, 6, 7, 8], np.uint64)
+    col = np.array([1, 2, 3, 4, 0, 0, 0, 0], np.uint32)
+    w = np.array(out_weights + back_weights, np.uint32)
+    G = ctx.graph(off, col, w, symmetric=True)
+    for s in range(5):
+        assert (G.mssssp(np.array([s], np.uint32))[0] == oracle.sssp(off, col, w, s)).all()
+    G.close()
