@@ -87,9 +87,10 @@ enum {
                                     BFS, hooking CC and pull PageRank on the same CSR */
     PTG_CSR_HOST_PINNED = 1u << 1, /* arrays already pinned (no registration needed) */
     PTG_CSR_WIDE_OFFSETS = 1u << 2 /* keep 64-bit offsets on the device even when
-                                      m < 2^32 (they are 64-bit anyway from 2^32
-                                      edges on, which the reference's u32 offsets
-                                      cannot hold, ptGraph/main.cu:99-102)         */
+                                      m < 2^32 (they are 64-bit anyway from 2^32 -
+                                      4096 edges on; from 2^32 on the reference's
+                                      u32 offsets cannot hold them,
+                                      ptGraph/main.cu:99-102)                      */
 };
 
 typedef struct ptg_csr {

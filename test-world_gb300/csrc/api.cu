@@ -539,7 +539,7 @@ ptg_status ptg_graph_create(ptg_ctx *ctx, const ptg_csr *csr, const ptg_partitio
         g->m = csr->m;
         g->symmetric = (csr->flags & PTG_CSR_SYMMETRIC) != 0;
         g->weighted = csr->weight != nullptr || csr->edges_aos != nullptr;
-        g->off64 = csr->m >= (1ull << 32) || (csr->flags & PTG_CSR_WIDE_OFFSETS) != 0;
+        g->off64 = wide_offsets(csr->m, csr->flags);
         // the caller's offsets are read in place (no host copy): the device
         // validation pass checks that they never decrease
         const HostOffsets off{csr->offsets, csr->offset_type == PTG_OFFSETS_U64,
@@ -1089,6 +1089,8 @@ void ptg_compat_set_partition_config(const ptg_partition_config *cfg) {
 }
 void ptg_compat_set_device(int device) { tls.device = device; }
 
+// For the tests: whether a graph of m edges gets 64-bit offsets.
+int ptg_internal_wide_offsets(uint64_t m, uint32_t flags) { return wide_offsets(m, flags); }
 // For the tests: how long a traversal's blocks wait at their barrier, and the host
 // for a level message.
 void ptg_internal_set_barrier_polls(ptg_ctx *ctx, uint64_t polls) {

@@ -1,7 +1,7 @@
 // ptg_internal.h - internal types of the GB300 graph engine (host + device).
 //
 // Layout in HBM (one ptg_graph):
-//   offsets   : OffT[n+1]   (u32 when m < 2^32, else u64; sentinel form)
+//   offsets   : OffT[n+1]   (u32 unless wide_offsets, else u64; sentinel form)
 //   col       : u32[resident_edges]      (structure of arrays)
 //   weight    : u32[resident_edges]      (weighted graphs only)
 // Edges past resident_edges stay in (pinned) host memory and stream through
@@ -352,6 +352,13 @@ namespace ptg {
 constexpr int kBlock = 256;
 constexpr int kItems = 8;
 constexpr int kTile = kBlock * kItems;  // edges per expand tile
+
+// Whether the offsets need 64 bits.  Loops over a row compare with its end an index
+// that may be a step past it (at most 32 lanes x 8 edges), which has to fit the
+// offset type as well.
+inline bool wide_offsets(uint64_t m, uint32_t flags) {
+    return m >= (1ull << 32) - 4096 || (flags & PTG_CSR_WIDE_OFFSETS) != 0;
+}
 
 void set_error(ptg_ctx *ctx, const Error &e);
 // Host->device copy of streamed edges [e0, e1) of h_col (which = 0) or h_w

@@ -587,7 +587,7 @@ ptg_status ptg_server_add_graph(ptg_server *s, ptg_graph *g, uint32_t *graph_id)
 ptg_status ptg_server_upload(ptg_server *s, const ptg_csr *csr, uint32_t *graph_id, uint32_t *resident) {
     if (!s || !csr || !graph_id) return PTG_ERR_INVALID;
     uint64_t bpe = (csr->weight || csr->edges_aos) ? 8 : 4;
-    uint64_t osz = (csr->offset_type == PTG_OFFSETS_U64 && csr->m >= (1ull << 32)) ? 8 : 4;
+    uint64_t osz = wide_offsets(csr->m, csr->flags) ? 8 : 4;
     uint64_t need = (csr->n + 1) * osz + csr->m * bpe;
     uint64_t left;
     {

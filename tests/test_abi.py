@@ -155,3 +155,13 @@ def test_default_partition_size_is_the_tuned_one(ptg):
     off = np.arange(0, (1 << 24) + 1, 4, dtype=np.uint64)  # 4M vertices of 4 edges, 16M edges
     P, R, PE, _ = ptg.plan_partitions(off, 8, 0, cfg)
     assert PE == (32 << 20) // 8 and P == (int(off[-1]) + PE - 1) // PE
+
+
+def test_offset_width_leaves_room_past_the_last_edge(ptg):
+    """32-bit offsets only where an index a few steps past the last edge still fits them."""
+    wide = ptg.lib().ptg_internal_wide_offsets
+    wide.argtypes = [ctypes.c_uint64, ctypes.c_uint32]
+    steps = 2 * 32 * 8
+    for m in (0, 1, 1 << 31, 2**32 - steps, 2**32 - 1, 2**32, 1 << 40):
+        assert wide(m, 0) == (m + steps >= 2**32)
+        assert wide(m, 4) == 1  # PTG_CSR_WIDE_OFFSETS
