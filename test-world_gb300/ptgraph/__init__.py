@@ -301,6 +301,9 @@ class Ctx:
         self.device = device
         self.h = _vp()
         self._deps = weakref.WeakSet()  # graphs and servers, closed before the context
+        # their handles (True: a server): a collector that finds a context and what
+        # depends on it in one cycle clears the weak references first
+        self._open = {}
         _check(lib().ptg_ctx_create(device, ctypes.byref(self.h)))
         _LIVE_CTX.add(self)
 
@@ -309,6 +312,9 @@ class Ctx:
             deps = list(self._deps)
             for d in sorted(deps, key=lambda d: not isinstance(d, Server)):  # servers before graphs
                 d.close()
+            for h, server in sorted(self._open.items(), key=lambda x: not x[1]):
+                (lib().ptg_server_destroy if server else lib().ptg_graph_destroy)(_vp(h))
+            self._open.clear()
             lib().ptg_ctx_destroy(self.h)
             self.h = _vp()
 
@@ -424,10 +430,12 @@ class Graph:
         _check(lib().ptg_graph_create(ctx.h, ctypes.byref(c), ctypes.byref(config) if config else None,
                                       ctypes.byref(self.h)), ctx.h)
         ctx._deps.add(self)
+        ctx._open[self.h.value] = False
 
     def close(self):
         if self.h:
-            lib().ptg_graph_destroy(self.h)
+            if self.ctx._open.pop(self.h.value, None) is not None:  # (else the context has closed it)
+                lib().ptg_graph_destroy(self.h)
             self.h = _vp()
 
     def __del__(self):
@@ -549,6 +557,7 @@ class Server:
         self.h = _vp()
         _check(lib().ptg_server_create(ctx.h, ctypes.byref(cfg), ctypes.byref(self.h)), ctx.h)
         ctx._deps.add(self)
+        ctx._open[self.h.value] = True
         self._keep = []      # graphs and uploaded arrays the server reads
         self._n = {}         # graph id -> vertices
         self._out = {}       # request id -> result buffer
@@ -615,7 +624,8 @@ class Server:
 
     def close(self):
         if self.h:
-            lib().ptg_server_destroy(self.h)
+            if self.ctx._open.pop(self.h.value, None) is not None:
+                lib().ptg_server_destroy(self.h)
             self.h = _vp()
 
     def __del__(self):

@@ -165,3 +165,37 @@ def test_offset_width_leaves_room_past_the_last_edge(ptg):
     for m in (0, 1, 1 << 31, 2**32 - steps, 2**32 - 1, 2**32, 1 << 40):
         assert wide(m, 0) == (m + steps >= 2**32)
         assert wide(m, 4) == 1  # PTG_CSR_WIDE_OFFSETS
+
+
+def test_collected_cycle_closes_the_context_last(ptg, monkeypatch):
+    """A context, a graph and a server that become garbage together: each is destroyed once, the
+    context last."""
+    import gc
+    real, log, count = ptg.lib(), [], [0]
+
+    class Fake:
+        def __getattr__(self, name):
+            def call(*args):
+                if name.endswith("_create"):
+                    count[0] += 1
+                    args[-1]._obj.value = count[0]
+                if name.endswith("_destroy"):
+                    log.append((name, args[0].value))
+                return 0
+            return call if name.endswith(("_create", "_destroy")) else getattr(real, name)
+
+    fake = Fake()
+    monkeypatch.setattr(ptg, "lib", lambda: fake)
+    for order in range(2):
+        log.clear()
+        count[0] = 0
+        c = ptg.Ctx(0)
+        g = c.graph(np.array([0, 1, 2], np.uint64), np.array([1, 0], np.uint32))
+        s = ptg.Server(c)
+        ring = [c, g, s] if order else [s, g, c]
+        for x in ring:
+            x.ring = ring
+        del c, g, s, ring, x
+        gc.collect()
+        assert sorted(log[:2]) == [("ptg_graph_destroy", 2), ("ptg_server_destroy", 3)]
+        assert log[2:] == [("ptg_ctx_destroy", 1)]
