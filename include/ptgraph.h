@@ -84,7 +84,10 @@ enum {
 };
 enum {
     PTG_CSR_SYMMETRIC = 1u << 0, /* every edge u->v has v->u: enables pull/bottom-up
-                                    BFS, hooking CC and pull PageRank on the same CSR */
+                                    BFS, hooking CC and pull PageRank on the same CSR.
+                                    Weights may differ between the two; SSSP rounds
+                                    pull where the first search finds them the same
+                                    (by sums of a hash with a random key)             */
     PTG_CSR_HOST_PINNED = 1u << 1, /* arrays already pinned (no registration needed) */
     PTG_CSR_WIDE_OFFSETS = 1u << 2 /* keep 64-bit offsets on the device even when
                                       m < 2^32 (they are 64-bit anyway from 2^32 -
@@ -171,8 +174,10 @@ typedef struct ptg_run_stats {
 
 typedef struct ptg_run_opts {
     uint32_t flags;             /* PTG_OUT_DEVICE | PTG_LEVEL_ZERO_BASED | ...     */
-    uint32_t delta;             /* SSSP near/far bucket width; 0 = auto            */
-    uint32_t max_iterations;    /* 0 = n + 1                                       */
+    uint32_t delta;             /* SSSP near/far bucket width; 0 = auto.  In HBM the
+                                   width of the first buckets: one that holds few
+                                   edges doubles the width of the next             */
+    uint32_t max_iterations;    /* 0 = 4 n + 16                                    */
     uint32_t reserved;
     ptg_run_stats *stats;       /* optional                                        */
 } ptg_run_opts;

@@ -8,18 +8,22 @@
 //   (PPR: r' = d * sum + [v == src] * ((1-d) + d * dangling))
 // with dangling = sum of r over zero-degree vertices and a fixed number of
 // iterations.  Ranks and contributions are stored in FP32; per-vertex sums
-// are compensated two-float sums (about 48 significant bits, beyond what the
-// 1e-6 tolerance needs), because GB300 runs FP32 adds at 64x its FP64 rate.
+// are compensated two-float sums, because GB300 runs FP32 adds at 64x its FP64
+// rate.  A lane collects the exact errors of its additions in one float (ff_term):
+// over the n <= 128 terms that a lane adds (pr_chunk / 32 where that is tuned up)
+// what is lost stays below about n^2 2^-48, 2^-34 of the sum, and the partials of
+// the lanes and pieces meet in renormalized two-floats.  The ranks are the same
+// bits as with a renormalization after each term.
 //
 // Pull over a symmetric CSR (in-edges == out-edges), as a degree-binned
 // SpMV: rows are grouped once per graph by degree (a thread, 8 lanes or a
-// warp per row, and warp-sized chunks of the longest rows), each lane keeps
+// warp per row, and warp-sized pieces of the longest rows), each lane keeps
 // its own two-float partial, and partials meet through shuffles in a fixed
-// order, so the result of a row does not depend on scheduling.  The bins of
-// an iteration run side by side on streams forked from the context stream
-// (they read the same input and write disjoint rows).  The gathered
-// contributions of a scale-24 graph (67 MB) stay in L2; DRAM carries the
-// column stream, so the gathers' L2 sector traffic is the bound.
+// order, so the result of a row does not depend on scheduling.  An iteration is
+// one launch: its warps take units of rows from counters, longest first, and
+// the warp that ends a long row's last piece adds the row's partial sums in
+// order.  The gathered contributions of a scale-24 graph (67 MB) stay in L2;
+// DRAM carries the column stream, so the gathers' L2 sector traffic is the bound.
 #include <algorithm>
 
 #include "ptg_device.cuh"
@@ -779,9 +783,10 @@ int pr_grid(ptg_graph *g, int ctas_per_sm, int sources, PrBins &bins) {
     const uint64_t units = bins.n_items + bins.big_units + bins.mid_units + bins.small_units;
     const int grid = grid_for(units, kBlock / 32, g->ctx->sm_count * per_sm);
     // From 2^27 edges on the units are long enough for one counter, which then
-    // balances best: 20 iterations of one source at RMAT-23 14.3 ms (16 slices:
-    // 15.1), at RMAT-22 6.8 (6.5), RMAT-18 0.95 (0.63).  A pass of several
-    // sources has longer units: RMAT-22 13.6 ms with 8 slices, 14.9 with 16.
+    // balances best: 20 iterations at RMAT-24 28.9 ms (16 slices: 29.0), RMAT-23
+    // 14.2 (15.0), RMAT-22 6.7 (6.3), RMAT-20 2.1 (1.5), RMAT-18 0.95 (0.63); of 8
+    // sources, whose units are longer, 59.3 (8 slices: 60.2), 28.0 (30.6), 13.5
+    // (13.6; 16 slices 15.0), 3.43 (3.29).
     bins.slices = std::min<unsigned>(g->m >= (1ull << 27) ? 1u : sources > 1 ? kSlices / 2 : kSlices, (unsigned)grid);
     return grid;
 }

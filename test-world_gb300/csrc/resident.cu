@@ -44,13 +44,14 @@
 // atomic.  Every wait at the barrier is bounded.
 //
 // What bounds it: a small graph's level is a chain of dependent reads and the
-// barrier, 5-10 us; the heavy SSSP rounds of RMAT-24 probe 190-290 G targets/s,
-// about what PageRank's gathers reach from L2 (one 32-byte sector each): the
-// round of 307 M edges took 1170 us as a push and takes 730 as a pull.  Staging the edges ahead with cp.async and dropping candidates by the largest
-// distance among the hubs changed neither.  Per search, before -> now: BFS on
-// RMAT-16 217 -> 87 us, on RMAT-24 580 -> 415 us; SSSP on RMAT-24 6.7 -> 3.2
-// ms; a served mix of small graphs 8.8 -> 6.5 ms (5.5 with PageRank's one launch
-// per iteration).
+// barrier, 5-10 us; the heavy SSSP rounds of RMAT-24 probe 150-260 G targets/s,
+// near what PageRank's gathers reach from L2 (one 32-byte sector each): a
+// round of 307 M edges took 1170 us as a push and takes 710 as a pull.  Staging
+// the edges ahead with cp.async and dropping candidates by the largest distance
+// among the hubs changed neither.  Per search, before -> now: BFS on RMAT-16 214
+// -> 83 us, on RMAT-24 590 -> 420 us; SSSP on RMAT-24 6.4-6.5 -> 3.2-3.7 ms (over
+// the machines that it was measured on); a served mix of small graphs 8.8 -> 6.5
+// ms (5.4 with PageRank's one launch per iteration).
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -71,9 +72,10 @@ constexpr int kBuWords = 16;    // frontier bitmap words per warp and pull step,
 constexpr unsigned kErrOverflow = 1u, kErrBarrier = 2u, kErrLimit = 4u;
 // SSSP buckets with fewer edges than this (or than half the vertices) double
 // the width of the next ones: such a bucket's two passes over the parked
-// vertices and its barriers (15 us, 100 us with 8 M parked) outweigh its
-// relaxations.  RMAT-24 from width 6: 24 rounds and 4.2 ms a search, 45 rounds
-// and 4.5 ms without.
+// vertices and its barriers (15 us, 60 us with 8 M parked) outweigh its
+// relaxations.  From width 6, with and without: RMAT-24 24 rounds and 3.48 ms a
+// search against 49 and 3.62, RMAT-22 1.13 against 1.35 ms, RMAT-20 0.60 against
+// 0.79, 4 K vertices 0.19 against 0.29.
 constexpr u64 kWideEdges = 1ull << 21;
 
 // Every thread takes the launch's decisions for itself, from words that it reads
@@ -698,6 +700,9 @@ __device__ void pull_phase(const ResArgs &a, const uint32_t *bm_cur, uint32_t *b
     buf_total(b, found, edges);
 }
 
+// 4 CTAs per SM: the rounds wait for reads, so warps count.  Push, pull and bucket
+// code share the 64 registers that leaves, and SSSP spills 144 bytes (stores; 180
+// of loads; 224 and 316 with 64-bit offsets), CC 28 and BFS 40.
 template <class OffT, int MODE>
 __global__ void __launch_bounds__(kBlock, 4) k_traverse(ResArgs a) {
     __shared__ uint32_t s_buf[kWarps][kBuf];

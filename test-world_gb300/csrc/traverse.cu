@@ -110,12 +110,6 @@ __device__ __forceinline__ void relax_probe(const PushTargets &t, uint32_t v, ui
     if (nd < t.value[v]) relax(t, v, nd, threshold);
 }
 
-// Build the frontier queue from its bitmap (a warp per 32 words, one atomic
-// per CTA step for the CTA's place in the queue: a per-warp atomic on the one
-// tail counter serialised dense levels) and take near vertices out of the far
-// pile (SSSP).
-
-
 // Vertex of set bit r of a warp's 32 bitmap words (word wd0 + lane in lane
 // `lane`, pre = inclusive popcount prefix over the lanes); every lane calls
 // it, each with its own r < the warp's total.
@@ -135,6 +129,10 @@ __device__ __forceinline__ uint32_t warp_bit_vertex(uint32_t word, uint32_t pre,
 __device__ __forceinline__ void compact_body(const uint32_t *bm, uint64_t words, uint32_t *q, TravCtl *ctl,
                                              uint32_t *far_bm);
 
+// Builds the frontier queue from its bitmap (a warp per 32 words, one atomic
+// per CTA step for the CTA's place in the queue: a per-warp atomic on the one
+// tail counter serialised dense levels) and takes near vertices out of the far
+// pile (SSSP).
 // `clear` (this level's frontier bitmap, read by nothing after this kernel)
 // is zeroed for reuse as the level after next's bitmap; with `advance` the
 // last CTA to finish ends the level: the next frontier's size becomes the
@@ -1099,9 +1097,11 @@ bool graph_weights_symmetric(ptg_graph *g) {
 // it as the graph shrinks.  Narrow buckets relax fewer edges twice, and their
 // number costs little since a bucket that holds few edges doubles the width of
 // the next ones; on a small graph a bucket is a few barriers either way.
-// RMAT-24 (5.2e8 edges, mean weight 32): 4.1 / 4.2 / 4.7 / 5.7 / 6.5 ms a
-// search at widths 4 / 6 / 12 / 24 / 96; RMAT-20: 0.71 / 0.72 / 0.75 / 0.78 /
-// 0.79; 4 K vertices: 0.26 ms at 6, 0.18 at 96.
+// Milliseconds a search at widths 4 / 6 / 12 / 24 / 96 (mean weight 32): RMAT-24 3.43
+// / 3.48 / 3.94 / 4.85 / 6.20, RMAT-22 1.09 / 1.13 / 1.35 / 1.41 / 1.71, RMAT-20
+// (2^24.9 edges) 0.58 / 0.60 / 0.58 / 0.61 / 0.62, 4 K vertices 0.20 / 0.19 / 0.19 / 0.18 /
+// 0.16.  Where the scale changes it matters little: 0.45 to 0.48 ms at any of them
+// with 2^23.9 and 2^24.4 edges, 0.37 to 0.42 (widest 0.36) with 2^22.9 and 2^23.4.
 uint32_t default_delta(ptg_graph *g) {
     const float tuned = g->ctx->tuning.sssp_delta_scale;
     if (!(tuned > 0.f)) return 0;  // label-correcting rounds
