@@ -36,9 +36,9 @@ void stream_edges(ptg_graph *g, int which, void *dst, uint64_t e0, uint64_t e1, 
     }
 }
 
-// Device address of h_col (which = 0) or h_w (1), or nullptr unless every
-// streamed partition in the page-locked range is mapped where the first one says.
-const uint32_t *mapped_edges(ptg_graph *g, int which) {
+// Where kernels read h_col (which = 0) or h_w (1): nowhere unless every streamed
+// partition in the page-locked range is mapped where the first one says.
+HostEdges mapped_edges(ptg_graph *g, int which) {
     const uint32_t *base = which ? g->h_w : g->h_col;
     const uintptr_t lo = std::max(g->pin_lo[which], (uintptr_t)(base + g->resident_edges));
     const uintptr_t hi = std::min(g->pin_hi[which], (uintptr_t)(base + g->m));
@@ -48,13 +48,31 @@ const uint32_t *mapped_edges(ptg_graph *g, int which) {
             void *d = nullptr;
             if (cudaHostGetDevicePointer(&d, (void *)x, 0) != cudaSuccess) {
                 cudaGetLastError();
-                return nullptr;
+                return {};
             }
             if (x == lo) shift = (uintptr_t)d - x;
-            if ((uintptr_t)d - x != shift) return nullptr;
+            if ((uintptr_t)d - x != shift) return {};
         }
     }
-    return lo < hi ? (const uint32_t *)((uintptr_t)base + shift) : nullptr;
+    if (lo >= hi) return {};
+    HostEdges h;
+    h.mid = (const uint32_t *)((uintptr_t)base + shift);
+    h.lo = (lo - (uintptr_t)base) / 4;
+    h.hi = (hi - (uintptr_t)base) / 4;
+    const uint64_t head = h.lo - g->resident_edges, tail = g->m - h.hi;
+    if (head + tail == 0) return h;
+    PinnedBuf &own = g->own_ends[which];
+    own.ensure((head + tail) * 4);
+    std::memcpy(own.p, base + g->resident_edges, head * 4);
+    std::memcpy(own.as<uint32_t>() + head, base + h.hi, tail * 4);
+    void *d = nullptr;
+    if (cudaHostGetDevicePointer(&d, own.p, 0) != cudaSuccess) {
+        cudaGetLastError();
+        return {};
+    }
+    h.head = (const uint32_t *)((uintptr_t)d - g->resident_edges * 4);
+    h.tail = (const uint32_t *)((uintptr_t)d + head * 4 - h.hi * 4);
+    return h;
 }
 
 void set_error(ptg_ctx *ctx, const Error &e) {
@@ -758,8 +776,8 @@ ptg_status ptg_graph_create(ptg_ctx *ctx, const ptg_csr *csr, const ptg_partitio
             }
             PTG_CUDA_TRY(cudaEventCreateWithFlags(&g->direct_done, cudaEventDisableTiming));
             PTG_CUDA_TRY(cudaEventCreateWithFlags(&g->hits_ready, cudaEventDisableTiming));
-            g->dev_col = mapped_edges(g, 0);
-            if (g->weighted) g->dev_w = mapped_edges(g, 1);
+            g->in_place[0] = mapped_edges(g, 0);
+            if (g->weighted) g->in_place[1] = mapped_edges(g, 1);
             g->device_bytes += (uint64_t)g->n_stage * PE * bpe;
             g->part_visits.assign(P, 0);
             if (g->cache_slots) {

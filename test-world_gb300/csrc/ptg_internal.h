@@ -290,6 +290,15 @@ struct HotSlot {
         if (freed) cudaEventDestroy(freed);
     }
 };
+
+// Streamed edges as kernels read them where they lie in host memory: edge x at
+// mid + x for x in [lo, hi), and before and after those (the caller's array has
+// parts of pages at its ends that cannot be page-locked) in copies at head + x and
+// tail + x.  mid == nullptr: they cannot.
+struct HostEdges {
+    const uint32_t *mid = nullptr, *head = nullptr, *tail = nullptr;
+    uint64_t lo = 0, hi = ~0ull;
+};
 }  // namespace ptg
 
 struct ptg_graph {
@@ -324,8 +333,8 @@ struct ptg_graph {
     const uint32_t *h_col = nullptr, *h_w = nullptr;  // pinned host edge arrays
     // page-locked address range of h_col / h_w (bytes outside it are pageable)
     uintptr_t pin_lo[2] = {0, 0}, pin_hi[2] = {~(uintptr_t)0, ~(uintptr_t)0};
-    // where kernels read h_col / h_w in place (by edge index; nullptr: they cannot)
-    const uint32_t *dev_col = nullptr, *dev_w = nullptr;
+    ptg::HostEdges in_place[2];                        // where kernels read h_col / h_w
+    ptg::PinnedBuf own_ends[2];                        // copies of their bytes that are not page-locked
     std::vector<void *> registered;                    // cudaHostRegister'ed ranges
     ptg::PinnedBuf own_col, own_w;                     // owned pinned copies
     ptg::DevBuf stage_col[3], stage_w[3];

@@ -374,6 +374,10 @@ __device__ __forceinline__ bool part_active(const uint32_t *bm_cur, const PushTa
     return bit_test(bm_cur, u) || (MODE != 0 && bit_test(t.bm_next, u));
 }
 
+__device__ __forceinline__ uint32_t ld_host(const HostEdges &h, uint64_t x) {
+    return __ldcs((x < h.lo ? h.head : x >= h.hi ? h.tail : h.mid) + x);
+}
+
 // Out-of-core: relaxes the frontier's streamed edges where they lie in host
 // memory, in the partitions that `direct` names, so that only their rows cross
 // the link.  Tiles of the scanned rows as k_expand, but a warp reads neighbouring
@@ -381,7 +385,7 @@ __device__ __forceinline__ bool part_active(const uint32_t *bm_cur, const PushTa
 // 160-200 GB/s on RMAT rows of 16 edges, where copies reach 211.
 template <class OffT, int MODE>
 __global__ void __launch_bounds__(kBlock) k_expand_host(const uint32_t *q, const OffT *sc, const OffT *rs,
-                                                        const uint32_t *tr, const uint32_t *col, const uint32_t *w,
+                                                        const uint32_t *tr, HostEdges col, HostEdges w,
                                                         const uint8_t *direct, uint64_t part_edges, PushTargets t) {
     const uint64_t E = t.ctl->E, ntiles = (E + kTile - 1) / kTile;
     const uint32_t thr = t.ctl->threshold;
@@ -405,8 +409,8 @@ __global__ void __launch_bounds__(kBlock) k_expand_host(const uint32_t *q, const
         }
 #pragma unroll
         for (int b = 0; b < kItems; b++) {
-            v[b] = e[b] != ~0ull ? __ldcs(col + e[b]) : PTG_UNREACHED;
-            nd[b] = MODE == 1 && e[b] != ~0ull ? __ldcs(w + e[b]) : 0u;
+            v[b] = e[b] != ~0ull ? ld_host(col, e[b]) : PTG_UNREACHED;
+            nd[b] = MODE == 1 && e[b] != ~0ull ? ld_host(w, e[b]) : 0u;
         }
 #pragma unroll
         for (int b = 0; b < kItems; b++) {
@@ -639,35 +643,15 @@ __global__ void __launch_bounds__(kBlock) k_far_split(uint32_t *far_bm, uint64_t
     }
 }
 
-// Whether a kernel may read the edges [e0, e1) in host memory.
-bool readable_in_place(const ptg_graph *g, uint64_t e0, uint64_t e1, bool weights) {
-    auto in = [&](int which, const uint32_t *h, const uint32_t *d) {
-        return d && (uintptr_t)(h + e0) >= g->pin_lo[which] && (uintptr_t)(h + e1) <= g->pin_hi[which];
-    };
-    return in(0, g->h_col, g->dev_col) && (!weights || in(1, g->h_w, g->dev_w));
-}
-
 // Hot-partition cache (the reference's visit-counted fragment promotion,
 // gpu_kernels.cu:254-282 and 475-485, where a 4096-edge fragment whose visit
 // record exceeds 3600 becomes a swap candidate).  part_visits[p] accumulates
 // the edges of frontier vertices that fell in partition p; a partition is hot
 // once that exceeds hot_threshold visits per 4096 edges.  A hot partition
-// takes a free slot, or the slot of the least worthy cached partition if it is
-// worthier itself; a cached partition is relaxed from its slot without a
+// takes a free slot, or the slot of the coldest cached partition if that one
+// has fewer visits; a cached partition is relaxed from its slot without a
 // copy, in this and every later traversal of the graph.
 //
-// A partition that kernels cannot read in place (the pages at the ends of the
-// caller's arrays are not page-locked) is copied whole for a single active
-// edge, so it is worthier than any that they can; else visits decide.
-bool less_worthy(const ptg_graph *g, uint64_t a, uint64_t b) {
-    auto in_place = [&](uint64_t p) {
-        const uint64_t e0 = p * g->partition_edges;
-        return readable_in_place(g, e0, std::min(g->m, e0 + g->partition_edges), g->weighted);
-    };
-    const bool ra = in_place(a), rb = in_place(b);
-    return ra != rb ? ra : g->part_visits[a] < g->part_visits[b];
-}
-
 // The slot that hot partition p may take in a round with these active edges per
 // partition, -1 if none: not one whose partition the round has yet to use.
 int hot_victim(const ptg_graph *g, uint64_t p, uint64_t edges, const unsigned long long *hits) {
@@ -678,9 +662,9 @@ int hot_victim(const ptg_graph *g, uint64_t p, uint64_t edges, const unsigned lo
         const int64_t q = g->slots[s].part;
         if (q < 0) return (int)s;
         if (hits[q] && (uint64_t)q > p) continue;
-        if (victim < 0 || less_worthy(g, q, g->slots[victim].part)) victim = (int)s;
+        if (victim < 0 || g->part_visits[q] < g->part_visits[g->slots[victim].part]) victim = (int)s;
     }
-    return victim >= 0 && less_worthy(g, g->slots[victim].part, p) ? victim : -1;
+    return victim >= 0 && g->part_visits[g->slots[victim].part] < g->part_visits[p] ? victim : -1;
 }
 
 // The slot of a partition that is copied now: its own, or one that it takes; -1
@@ -907,13 +891,14 @@ void traverse_impl(ptg_graph *g, TravKind kind, uint32_t src, uint32_t *d_value,
             // (never, 1/4, 1/2, 3/4, 7/8, always): RMAT-22 half streamed 10.9,
             // 6.2, 4.9, 4.8, 4.8, 5.2 ms; RMAT-24 all streamed 55, 26.6, 21.9,
             // 21.4, 21.4, 23.3 ms; BFS of the former 4.5, 2.0, 1.9, 1.9, 1.9, 1.9.
+            const bool readable = g->in_place[0].mid && (!need_w || g->in_place[1].mid);
             uint64_t active = 0, direct = 0;  // streamed edges of the frontier; those read in place
             uint64_t spared = 0;              // edges that are not copied for that
             for (uint64_t p = g->resident_partitions; p < P && hot; p++) g->part_visits[p] += h_hits[p];
             for (uint64_t p = g->resident_partitions; p < P; p++) {
                 const uint64_t e0 = p * g->partition_edges, e1 = std::min<uint64_t>(g->m, e0 + g->partition_edges);
                 // (what is in a cache slot, or is copied into one now, needs no link)
-                h_direct[p] = h_hits[p] && h_hits[p] * 4 <= (e1 - e0) * 3 && readable_in_place(g, e0, e1, need_w) &&
+                h_direct[p] = h_hits[p] && h_hits[p] * 4 <= (e1 - e0) * 3 && readable &&
                               !(hot && sparse_slot(g, p, e1 - e0, h_hits));
                 rr.parts_skipped += !h_hits[p];
                 active += h_hits[p];
@@ -940,13 +925,13 @@ void traverse_impl(ptg_graph *g, TravKind kind, uint32_t src, uint32_t *d_value,
                 const int hg = grid_for(active, kTile, sms * 8);
                 if (kind == TRAV_BFS)
                     launch(ctx, "k_expand_host_bfs", k_expand_host<OffT, 0>, hg, kBlock, 0, st, q_cur, sc, rs, tr,
-                           g->dev_col, g->dev_w, d_direct, g->partition_edges, pt);
+                           g->in_place[0], g->in_place[1], d_direct, g->partition_edges, pt);
                 else if (kind == TRAV_SSSP)
                     launch(ctx, "k_expand_host_sssp", k_expand_host<OffT, 1>, hg, kBlock, 0, st, q_cur, sc, rs, tr,
-                           g->dev_col, g->dev_w, d_direct, g->partition_edges, pt);
+                           g->in_place[0], g->in_place[1], d_direct, g->partition_edges, pt);
                 else
                     launch(ctx, "k_expand_host_cc", k_expand_host<OffT, 2>, hg, kBlock, 0, st, q_cur, sc, rs, tr,
-                           g->dev_col, g->dev_w, d_direct, g->partition_edges, pt);
+                           g->in_place[0], g->in_place[1], d_direct, g->partition_edges, pt);
                 PTG_CUDA_TRY(cudaGetLastError());
                 PTG_CUDA_TRY(cudaEventRecord(g->direct_done, st));
                 rr.link_bytes += direct * (need_w ? 8 : 4);

@@ -69,3 +69,35 @@ def test_sparse_rounds_fill_the_hot_cache(ptg, ctx, oracle, slots, host):
     if slots == 64:
         assert second["link_bytes"] * 5 < first["link_bytes"]
     G.close()
+
+
+@pytest.mark.parametrize("shift", [(0, 0), (1, 0), (0, 1023), (700, 3)])
+@pytest.mark.parametrize("policy", ["PREFIX", "NONE"])
+@pytest.mark.parametrize("name,length", [("chain", 20000), ("hubs", 0)])
+def test_ends_that_cannot_be_page_locked(ptg, ctx, oracle, shift, policy, name, length):
+    """Pageable arrays that begin and end somewhere in a page: the edges of the partial pages are read
+    in place as well, from the first and last partition too."""
+    n, src, dst, s = chain(length, 4) if length else hubs([5000, 9000, 20000, 40000], 2)
+    off, col, w = csr(n, src, dst, True, n)
+    m = col.size
+
+    def place(a, at):
+        room = np.zeros(m + (1 << 15) + at, np.uint32)  # (of its own: no page shared with another array)
+        first = -(room.ctypes.data // 4) % (1 << 14) + at  # `at` words behind a 64 KB boundary
+        room[first:first + m] = a
+        return room[first:first + m]
+
+    col, w = place(col, shift[0]), place(w, shift[1])
+    cfg = ptg.partition_config(partition_bytes=1 << 15, device_budget_bytes=3 << 15, force_out_of_core=1,
+                               resident_policy=getattr(ptg, "PTG_RESIDENT_" + policy))
+    G = ctx.graph(off, col, w, symmetric=False, config=cfg)
+    st = {}
+    assert (G.bfs(s, stats=st) == oracle.bfs(off, col, s, method="queue")).all()
+    if name == "chain":  # a vertex a round: its edges, not its partition
+        assert st["link_bytes"] <= 4 * m
+    assert (G.sssp(s, stats=st) == oracle.sssp(off, col, w, s)).all()
+    if name == "chain":
+        assert st["link_bytes"] <= 8 * m
+    else:
+        assert (G.cc() == oracle.cc(off, col)).all()
+    G.close()
